@@ -1010,7 +1010,7 @@ clb_status ade_init(clb_handle* h, const clb_species_desc* sp, int S) {
     for (int i = 0; i < S; ++i) {
         if (P.mobile[i]) continue;
         std::fill(immh.begin(), immh.end(), P.c0[i]);
-        cudaMemcpy(h->d_imm + (size_t)i * N1, immh.data(), sizeof(double) * N1, cudaMemcpyHostToDevice);
+        copy_on_stream(h, h->d_imm + (size_t)i * N1, immh.data(), sizeof(double) * N1, cudaMemcpyHostToDevice);
     }
     // stored boundary densities: Dirichlet value, else c0 (lattice.initialize() runs the
     // Neumann processor once on the equilibrium field)
@@ -1022,14 +1022,14 @@ clb_status ade_init(clb_handle* h, const clb_species_desc* sp, int S) {
             std::fill(neu.begin() + ((size_t)i * 2 + side) * h->g.plane,
                       neu.begin() + ((size_t)i * 2 + side + 1) * h->g.plane, v);
         }
-    cudaMemcpy(h->d_neu, neu.data(), sizeof(double) * neu.size(), cudaMemcpyHostToDevice);
+    copy_on_stream(h, h->d_neu, neu.data(), sizeof(double) * neu.size(), cudaMemcpyHostToDevice);
     int mt[16] = {0};
     for (size_t k = 0; k < mob.size(); ++k) mt[k] = mob[k];
-    cudaMemcpy(mob_table(h), mt, sizeof(mt), cudaMemcpyHostToDevice);
+    copy_on_stream(h, mob_table(h), mt, sizeof(mt), cudaMemcpyHostToDevice);
     if (!c0m.empty()) {
         double* dc0 = nullptr;
         cudaMalloc(&dc0, sizeof(double) * c0m.size());
-        cudaMemcpy(dc0, c0m.data(), sizeof(double) * c0m.size(), cudaMemcpyHostToDevice);
+        copy_on_stream(h, dc0, c0m.data(), sizeof(double) * c0m.size(), cudaMemcpyHostToDevice);
         const int grid = h->num_sms * 8;
         switch (h->ade_prec) {
             case CLB_F64: k_ade_init<double><<<grid, 256, 0, h->stream>>>((double*)h->d_g, (double*)h->d_glink, (int64_t)KS, L, (int64_t)SSz, h->n_mobile, dc0); break;
@@ -1134,7 +1134,7 @@ clb_status ade_set_immobile(clb_handle* h, int s, const double* host) {
     if (s < 0 || s >= h->S) return fail(h, CLB_INVALID_ARG, "species index out of range");
     const int si = h->u2i[s];
     if (h->ap.slot[si] >= 0) return fail(h, CLB_INVALID_ARG, "not an immobile species");
-    return cuda_check(h, cudaMemcpy(h->d_imm + (size_t)si * h->g.N, host, sizeof(double) * (size_t)h->g.N,
+    return cuda_check(h, copy_on_stream(h, h->d_imm + (size_t)si * h->g.N, host, sizeof(double) * (size_t)h->g.N,
                                     cudaMemcpyHostToDevice), "immobile concentration");
 }
 
@@ -1220,7 +1220,7 @@ clb_status ade_set_biomass(clb_handle* h, int M, const double* b) {
     if (M == 0) return CLB_OK;
     cudaError_t e = cudaMalloc(&h->d_bio, sizeof(double) * M * (size_t)h->g.N);
     if (e != cudaSuccess) return cuda_check(h, e, "biomass");
-    clb_status st = cuda_check(h, cudaMemcpy(h->d_bio, b, sizeof(double) * M * (size_t)h->g.N, cudaMemcpyHostToDevice),
+    clb_status st = cuda_check(h, copy_on_stream(h, h->d_bio, b, sizeof(double) * M * (size_t)h->g.N, cudaMemcpyHostToDevice),
                                "biomass copy");
     return st == CLB_OK ? refresh_bflag(h) : st;
 }
@@ -1782,7 +1782,7 @@ clb_status ade_set_populations(clb_handle* h, int s, const double* host, int shi
     double* buf = nullptr;
     cudaError_t e = cudaMalloc(&buf, sizeof(double) * 7 * (size_t)h->g.N);
     if (e != cudaSuccess) return cuda_check(h, e, "population buffer");
-    cudaMemcpy(buf, host, sizeof(double) * 7 * (size_t)h->g.N, cudaMemcpyHostToDevice);
+    copy_on_stream(h, buf, host, sizeof(double) * 7 * (size_t)h->g.N, cudaMemcpyHostToDevice);
     const int odd = (int)(h->ade_iters & 1);
     const int grid = h->num_sms * 8;
     const size_t off = (size_t)m * h->ade_sp.SS, loff = off;
@@ -1806,7 +1806,7 @@ clb_status ade_density(clb_handle* h, int s, double* host) {
     s = h->u2i[s];
     const size_t N = (size_t)h->g.N;
     if (h->ap.slot[s] < 0)
-        return cuda_check(h, cudaMemcpy(host, h->d_imm + (size_t)s * N, sizeof(double) * N, cudaMemcpyDeviceToHost), "immobile copy");
+        return cuda_check(h, copy_on_stream(h, host, h->d_imm + (size_t)s * N, sizeof(double) * N, cudaMemcpyDeviceToHost), "immobile copy");
     // the Neumann planes' stored values as the reference holds them after the last stream
     refresh_neumann(h);
     if (!h->d_stage) {
@@ -1836,14 +1836,14 @@ clb_status ade_density(clb_handle* h, int s, double* host) {
 clb_status ade_biomass(clb_handle* h, int m, double* host) {
     if (!h->ade_ready || m < 0 || m >= h->M) return fail(h, CLB_INVALID_ARG, "no such biomass field");
     h->ca_full = true;
-    return cuda_check(h, cudaMemcpy(host, h->d_bio + (size_t)m * h->g.N, sizeof(double) * h->g.N, cudaMemcpyDeviceToHost), "biomass copy");
+    return cuda_check(h, copy_on_stream(h, host, h->d_bio + (size_t)m * h->g.N, sizeof(double) * h->g.N, cudaMemcpyDeviceToHost), "biomass copy");
 }
 
 clb_status ade_set_biomass_field(clb_handle* h, int m, const double* host) {
     if (!h->ade_ready || m < 0 || m >= h->M) return fail(h, CLB_INVALID_ARG, "no such biomass field");
     h->ca_full = true;
     clb_status st = cuda_check(
-        h, cudaMemcpy(h->d_bio + (size_t)m * h->g.N, host, sizeof(double) * h->g.N, cudaMemcpyHostToDevice), "biomass copy");
+        h, copy_on_stream(h, h->d_bio + (size_t)m * h->g.N, host, sizeof(double) * h->g.N, cudaMemcpyHostToDevice), "biomass copy");
     return st == CLB_OK ? refresh_bflag(h) : st;
 }
 

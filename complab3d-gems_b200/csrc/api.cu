@@ -31,7 +31,7 @@ clb_status cuda_check(clb_handle* h, cudaError_t e, const char* what) {
 // moves no map to the host in iterations where nobody reads it.
 clb_status host_mat_sync(clb_handle* h) {
     if (!h->h_mat_stale) return CLB_OK;
-    cudaError_t e = cudaMemcpy(h->h_mat.data(), h->d_mat, (size_t)h->g.N, cudaMemcpyDeviceToHost);
+    cudaError_t e = copy_on_stream(h, h->h_mat.data(), h->d_mat, (size_t)h->g.N, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_check(h, e, "material copy");
     h->h_mat_stale = false;
     return CLB_OK;
@@ -92,7 +92,7 @@ clb_status clb_create(const clb_domain_desc* desc, const int8_t* material, clb_h
     h->h_mat.assign(material, material + N);
     cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&h->d_mat, N);
-    if (e == cudaSuccess) e = cudaMemcpy(h->d_mat, material, N, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = copy_on_stream(h, h->d_mat, material, N, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         std::string m = std::string("create: ") + cudaGetErrorString(e);
         if (h->d_mat) cudaFree(h->d_mat);
@@ -133,7 +133,7 @@ clb_status clb_synchronize(clb_handle* h) {
     if (s != CLB_OK) return s;
     if (!h->d_err) return ade_nonfinite_check(h);
     int flag = 0;
-    cudaMemcpy(&flag, h->d_err, sizeof(int), cudaMemcpyDeviceToHost);
+    copy_on_stream(h, &flag, h->d_err, sizeof(int), cudaMemcpyDeviceToHost);
     if (flag) return fail(h, CLB_TIMEOUT, "a bounded device wait gave up (bulk copy did not complete)");
     return ade_nonfinite_check(h);
 }

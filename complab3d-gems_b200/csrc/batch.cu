@@ -217,6 +217,8 @@ clb_status batch_create(clb_handle* const* hs, int n, clb_batch** out) {
     if (e == cudaSuccess && !jobs.empty())
         e = cudaMemcpy(b->d_jobs, jobs.data(), sizeof(NeumannJob) * jobs.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(b->d_joff, joff.data(), sizeof(int64_t) * joff.size(), cudaMemcpyHostToDevice);
+    // the batch's own stream does not wait for the legacy stream's uploads
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
     if (e != cudaSuccess) {
         batch_free(b);
         delete b;
@@ -285,6 +287,7 @@ static clb_status persist_table(clb_batch* b, int steps, bool flow, bool ade, cl
     if (e == cudaSuccess && !items.empty())
         e = cudaMemcpy(t.items, items.data(), sizeof(BatchItem) * items.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(t.need, need.data(), sizeof(int) * need.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
     if (e != cudaSuccess) {
         cudaFree(t.items);
         cudaFree(t.need);

@@ -1000,7 +1000,7 @@ clb_status ca_setup(clb_handle* h, const clb_ca_desc* d) {
         // from now on the mask moves with the automaton; the flow keeps its own map until a refresh
         h->h_mat_flow = h->h_mat;
         e = cudaMalloc(&h->d_mat_flow, N);
-        if (e == cudaSuccess) e = cudaMemcpy(h->d_mat_flow, h->h_mat_flow.data(), N, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = copy_on_stream(h, h->d_mat_flow, h->h_mat_flow.data(), N, cudaMemcpyHostToDevice);
         if (e != cudaSuccess) return cuda_check(h, e, "flow material map");
     }
     h->ca_bmax = d->max_biomass;
@@ -1137,7 +1137,7 @@ clb_status refresh_dynamics(clb_handle* h, int species, int flow) {
             h->h_mat_flow = h->h_mat;
             e = cudaMalloc(&h->d_mat_flow, (size_t)N);
             if (e == cudaSuccess)
-                e = cudaMemcpy(h->d_mat_flow, h->h_mat_flow.data(), (size_t)N, cudaMemcpyHostToDevice);
+                e = copy_on_stream(h, h->d_mat_flow, h->h_mat_flow.data(), (size_t)N, cudaMemcpyHostToDevice);
             if (e != cudaSuccess) return cuda_check(h, e, "flow material map");
         }
         h->launches += 2;
@@ -1169,10 +1169,10 @@ clb_status ca_fields(clb_handle* h, int which, double* host) {
     const size_t N = (size_t)h->g.N;
     cudaError_t e;
     if (which == 0) {
-        e = cudaMemcpy(host, h->d_ca_total, sizeof(double) * N, cudaMemcpyDeviceToHost);
+        e = copy_on_stream(h, host, h->d_ca_total, sizeof(double) * N, cudaMemcpyDeviceToHost);
     } else {
         std::vector<int> a(N);
-        e = cudaMemcpy(a.data(), h->d_ca_age, sizeof(int) * N, cudaMemcpyDeviceToHost);
+        e = copy_on_stream(h, a.data(), h->d_ca_age, sizeof(int) * N, cudaMemcpyDeviceToHost);
         for (size_t n = 0; n < N; ++n) host[n] = a[n];
     }
     return cuda_check(h, e, "automaton field");

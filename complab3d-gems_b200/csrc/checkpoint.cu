@@ -187,7 +187,7 @@ clb_status clb_checkpoint_load(clb_handle* h, const char* path) {
         Tracer tz;
         std::memset(&tz, 0, sizeof(tz));
         tz.iterations = hd.flow_iters;
-        cudaError_t e = cudaMemcpy(h->d_tracer, &tz, sizeof(tz), cudaMemcpyHostToDevice);
+        cudaError_t e = copy_on_stream(h, h->d_tracer, &tz, sizeof(tz), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) { h->flow_iters = save_flow; return cuda_check(h, e, "tracer"); }
         if ((st = clb_set_field(h, CLB_FIELD_FLOW_POPULATIONS, 0, flow.data(), 0)) != CLB_OK) return st;
     }

@@ -343,6 +343,13 @@ clb_status fail(clb_handle* h, clb_status s, const std::string& msg);
 // brings h_mat up to date with the device map after automaton passes changed it (api.cu)
 clb_status host_mat_sync(clb_handle* h);
 clb_status cuda_check(clb_handle* h, cudaError_t e, const char* what);
+// A copy in the order of the handle's stream, completed on return. (A plain cudaMemcpy belongs to the
+// legacy stream, which the handle's non-blocking stream neither waits for nor is waited for by: an
+// upload from pageable memory may still be on its way when it returns.)
+inline cudaError_t copy_on_stream(clb_handle* h, void* dst, const void* src, size_t bytes, cudaMemcpyKind kind) {
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, kind, h->stream);
+    return e == cudaSuccess ? cudaStreamSynchronize(h->stream) : e;
+}
 
 // flow.cu
 clb_status flow_init(clb_handle* h, double delta_p);

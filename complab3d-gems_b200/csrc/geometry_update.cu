@@ -241,11 +241,11 @@ clb_status geometry_refresh(clb_handle* h) {
     const bool need_lists = P.law2 != CLB_LAW_NONE || P.dis_on;
     if (!need_iface && !need_lists) return CLB_OK;
     std::vector<int32_t> node((size_t)K);
-    cudaError_t e = cudaMemcpy(node.data(), h->ade_sp.node, sizeof(int32_t) * K, cudaMemcpyDeviceToHost);
+    cudaError_t e = copy_on_stream(h, node.data(), h->ade_sp.node, sizeof(int32_t) * K, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_check(h, e, "node list");
     std::vector<uint8_t> stamp((size_t)G.N, 0);
     if (h->d_stamp) {
-        e = cudaMemcpy(stamp.data(), h->d_stamp, (size_t)G.N, cudaMemcpyDeviceToHost);
+        e = copy_on_stream(h, stamp.data(), h->d_stamp, (size_t)G.N, cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) return cuda_check(h, e, "stamp field");
     }
     const std::vector<int8_t>& mat = h->h_mat;
@@ -292,8 +292,8 @@ clb_status geometry_refresh(clb_handle* h) {
         if ((st = grow(h, (void**)&h->d_iface, (size_t)std::max<int64_t>(K, 1), "surface gate")) != CLB_OK) return st;
         if ((st = grow(h, (void**)&h->d_xidx, sizeof(int32_t) * std::max<int64_t>(K, 1), "gather index")) != CLB_OK) return st;
     }
-    cudaMemcpy(h->d_iface, iface.data(), iface.size(), cudaMemcpyHostToDevice);
-    cudaMemcpy(h->d_xidx, xidx.data(), sizeof(int32_t) * xidx.size(), cudaMemcpyHostToDevice);
+    copy_on_stream(h, h->d_iface, iface.data(), iface.size(), cudaMemcpyHostToDevice);
+    copy_on_stream(h, h->d_xidx, xidx.data(), sizeof(int32_t) * xidx.size(), cudaMemcpyHostToDevice);
     const int S = h->S;
     if ((int64_t)seal.size() > h->seal_cap || !h->d_seal) {
         h->seal_cap = std::max<int64_t>((int64_t)seal.size() * 2, 256);
@@ -308,10 +308,10 @@ clb_status geometry_refresh(clb_handle* h) {
     }
     h->n_seal = (int64_t)seal.size();
     h->n_gath = (int64_t)gath.size();
-    if (!seal.empty()) cudaMemcpy(h->d_seal, seal.data(), sizeof(int32_t) * seal.size(), cudaMemcpyHostToDevice);
+    if (!seal.empty()) copy_on_stream(h, h->d_seal, seal.data(), sizeof(int32_t) * seal.size(), cudaMemcpyHostToDevice);
     if (!gath.empty()) {
-        cudaMemcpy(h->d_gath, gath.data(), sizeof(int32_t) * gath.size(), cudaMemcpyHostToDevice);
-        cudaMemcpy(h->d_gath_nb, gnb.data(), sizeof(int32_t) * gnb.size(), cudaMemcpyHostToDevice);
+        copy_on_stream(h, h->d_gath, gath.data(), sizeof(int32_t) * gath.size(), cudaMemcpyHostToDevice);
+        copy_on_stream(h, h->d_gath_nb, gnb.data(), sizeof(int32_t) * gnb.size(), cudaMemcpyHostToDevice);
     }
     return cuda_check(h, cudaGetLastError(), "geometry lists");
 }
@@ -416,7 +416,7 @@ clb_status precip_setup(clb_handle* h, const clb_precip_desc* d) {
 static clb_status flow_follow(clb_handle* h) {
     const int64_t N = h->g.N;
     std::vector<uint8_t> stamp((size_t)N);
-    cudaError_t e = cudaMemcpy(stamp.data(), h->d_stamp, (size_t)N, cudaMemcpyDeviceToHost);
+    cudaError_t e = copy_on_stream(h, stamp.data(), h->d_stamp, (size_t)N, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_check(h, e, "stamp field");
     h->h_mat_flow = h->h_mat;
     for (int64_t n = 0; n < N; ++n)
@@ -425,7 +425,7 @@ static clb_status flow_follow(clb_handle* h) {
         e = cudaMalloc(&h->d_mat_flow, (size_t)N);
         if (e != cudaSuccess) return cuda_check(h, e, "flow material map");
     }
-    e = cudaMemcpy(h->d_mat_flow, h->h_mat_flow.data(), (size_t)N, cudaMemcpyHostToDevice);
+    e = copy_on_stream(h, h->d_mat_flow, h->h_mat_flow.data(), (size_t)N, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_check(h, e, "flow material map");
     ++h->launches;
     k_flow_codes<<<h->num_sms * 4, 256, 0, h->stream>>>(h->flow_sp.code, h->flow_sp.node, h->flow_sp.K, h->d_mat_flow);
@@ -465,10 +465,10 @@ clb_status geometry_update(clb_handle* h, int* sealed, int* reopened) {
         h->h_mat_flow = h->h_mat;
         e = cudaMalloc(&h->d_mat_flow, (size_t)h->g.N);
         if (e == cudaSuccess)
-            e = cudaMemcpy(h->d_mat_flow, h->h_mat_flow.data(), (size_t)h->g.N, cudaMemcpyHostToDevice);
+            e = copy_on_stream(h, h->d_mat_flow, h->h_mat_flow.data(), (size_t)h->g.N, cudaMemcpyHostToDevice);
         if (e != cudaSuccess) return cuda_check(h, e, "flow material map");
     }
-    e = cudaMemcpy(h->h_mat.data(), h->d_mat, (size_t)h->g.N, cudaMemcpyDeviceToHost);
+    e = copy_on_stream(h, h->h_mat.data(), h->d_mat, (size_t)h->g.N, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_check(h, e, "material copy");
     h->h_mat_stale = false;
     clb_status st = geometry_refresh(h);

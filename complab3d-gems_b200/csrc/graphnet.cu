@@ -255,7 +255,7 @@ clb_status graphnet_set(clb_handle* h, const char* path, const char* const* spec
         if (err != cudaSuccess) return cuda_check(h, err, "graph networks");
     }
     const int slot = abiotic ? CLB_MAX_MICROBES : microbe;
-    cudaError_t err = cudaMemcpy(static_cast<GnnNet*>(h->d_gnn) + slot, &N, sizeof N, cudaMemcpyHostToDevice);
+    cudaError_t err = copy_on_stream(h, static_cast<GnnNet*>(h->d_gnn) + slot, &N, sizeof N, cudaMemcpyHostToDevice);
     if (err != cudaSuccess) return cuda_check(h, err, "graph network");
     if (!h->gnn_host) h->gnn_host = new GnnNet[SYM_MAX_PROGS];
     h->gnn_host[slot] = N;

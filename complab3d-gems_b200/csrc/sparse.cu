@@ -275,7 +275,7 @@ clb_status sparse_build(clb_handle* h, const int8_t* stored_by_code, int q, Spar
         k_sb_words<<<blocks_for(RW), SB_THREADS, 0, st>>>(dmat, T, R, nz, W, out.rowmask, wcount);
         e = scan_exclusive(wcount, wcount, RW, scal, st);  // wcount now holds the word prefixes
     }
-    if (e == cudaSuccess) e = cudaMemcpy(&hs[0], scal, sizeof(int32_t), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = copy_on_stream(h, &hs[0], scal, sizeof(int32_t), cudaMemcpyDeviceToHost);
     const int64_t K = hs[0];
     if (e == cudaSuccess) e = cudaMalloc(&out.rowstart, sizeof(int32_t) * std::max(1, R));
     if (e == cudaSuccess) e = cudaMalloc(&out.rowpre, sizeof(int32_t) * RW);
@@ -296,7 +296,7 @@ clb_status sparse_build(clb_handle* h, const int8_t* stored_by_code, int q, Spar
         if (q == 19) k_sb_wall<19><<<blocks_for(K), SB_THREADS, 0, st>>>(out.node, out.idx_of, K, G, out.wall, edge, lcount);
         else k_sb_wall<7><<<blocks_for(K), SB_THREADS, 0, st>>>(out.node, out.idx_of, K, G, out.wall, edge, lcount);
         e = scan_exclusive(lcount, out.linkbase, K, scal + 1, st);
-        if (e == cudaSuccess) e = cudaMemcpy(&hs[1], scal + 1, sizeof(int32_t), cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess) e = copy_on_stream(h, &hs[1], scal + 1, sizeof(int32_t), cudaMemcpyDeviceToHost);
     }
     const int64_t L = hs[1];
     const int64_t T_ = std::max<int64_t>(1, (K + TILE - 1) / TILE);

@@ -1167,7 +1167,7 @@ clb_status surrogate_train(clb_handle* h, const clb_surrogate_train_desc* d, clb
         if (val < best_val) {
             best_val = val;
             since = 0;
-            cudaMemcpy(best.data(), P, sizeof(float) * P_N, cudaMemcpyDeviceToHost);
+            copy_on_stream(h, best.data(), P, sizeof(float) * P_N, cudaMemcpyDeviceToHost);
         } else if (++since >= d->patience) {
             ++epoch;
             break;

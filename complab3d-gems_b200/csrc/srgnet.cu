@@ -226,7 +226,7 @@ clb_status srg_set(clb_handle* h, const char* path, const char* const* species_n
         cudaError_t err = cudaMalloc(&h->d_srg, sizeof(SrgNet) * CLB_MAX_MICROBES);
         if (err != cudaSuccess) return cuda_check(h, err, "surrogate networks");
     }
-    cudaError_t err = cudaMemcpy(static_cast<SrgNet*>(h->d_srg) + microbe, &N, sizeof N, cudaMemcpyHostToDevice);
+    cudaError_t err = copy_on_stream(h, static_cast<SrgNet*>(h->d_srg) + microbe, &N, sizeof N, cudaMemcpyHostToDevice);
     if (err != cudaSuccess) return cuda_check(h, err, "surrogate network");
     if (!h->srg_host) h->srg_host = new SrgNet[CLB_MAX_MICROBES];
     h->srg_host[microbe] = N;

@@ -396,7 +396,7 @@ clb_status symbolic_set(clb_handle* h, const char* path, const char* const* spec
         if (err != cudaSuccess) return cuda_check(h, err, "rate-law programs");
     }
     const int slot = abiotic ? CLB_MAX_MICROBES : microbe;
-    cudaError_t err = cudaMemcpy(static_cast<SymProg*>(h->d_sym) + slot, &P, sizeof P, cudaMemcpyHostToDevice);
+    cudaError_t err = copy_on_stream(h, static_cast<SymProg*>(h->d_sym) + slot, &P, sizeof P, cudaMemcpyHostToDevice);
     if (err != cudaSuccess) return cuda_check(h, err, "rate-law program");
     h->sym_host[slot] = P;
     AdeParams& A = h->ap;
