@@ -343,12 +343,15 @@ clb_status fail(clb_handle* h, clb_status s, const std::string& msg);
 // brings h_mat up to date with the device map after automaton passes changed it (api.cu)
 clb_status host_mat_sync(clb_handle* h);
 clb_status cuda_check(clb_handle* h, cudaError_t e, const char* what);
-// A copy in the order of the handle's stream, completed on return. (A plain cudaMemcpy belongs to the
-// legacy stream, which the handle's non-blocking stream neither waits for nor is waited for by: an
-// upload from pageable memory may still be on its way when it returns.)
+// A copy after everything on the handle's stream and before everything that follows, completed on
+// return. (A plain cudaMemcpy belongs to the legacy stream, which the handle's non-blocking stream
+// neither waits for nor is waited for by, and an upload from pageable memory may still be on its way
+// when it returns. It is what moves pageable memory fastest, so it stays, with both waits.)
 inline cudaError_t copy_on_stream(clb_handle* h, void* dst, const void* src, size_t bytes, cudaMemcpyKind kind) {
-    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, kind, h->stream);
-    return e == cudaSuccess ? cudaStreamSynchronize(h->stream) : e;
+    cudaError_t e = cudaStreamSynchronize(h->stream);
+    if (e == cudaSuccess) e = cudaMemcpy(dst, src, bytes, kind);
+    if (e == cudaSuccess && kind == cudaMemcpyHostToDevice) e = cudaStreamSynchronize(cudaStreamLegacy);
+    return e;
 }
 
 // flow.cu
