@@ -1,5 +1,7 @@
 // ade.cu -- every species' D3Q7 advection-diffusion lattice, the kinetics and the deposit
-// in one fused pass per transport step.
+// in one fused pass per transport step. The step here stages a node's species in shared memory, for
+// laws that couple them (abiotic laws, dissolution, the thermodynamic gate, rate-law files); the
+// compiled biotic laws alone run the streamed step of ade_stream.cu.
 //
 // Reference behaviour (complab.cpp:2307-2315 collide, :2340-2452 run_kinetics +
 // update_rxnLattices, :3251-3259 stream; complab_functions.hh:347-442 soluteDomainSetup):
@@ -28,6 +30,7 @@
 #include <algorithm>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 namespace clb {
 
@@ -1134,8 +1137,8 @@ clb_status ade_set_immobile(clb_handle* h, int s, const double* host) {
     if (s < 0 || s >= h->S) return fail(h, CLB_INVALID_ARG, "species index out of range");
     const int si = h->u2i[s];
     if (h->ap.slot[si] >= 0) return fail(h, CLB_INVALID_ARG, "not an immobile species");
-    return cuda_check(h, copy_on_stream(h, h->d_imm + (size_t)si * h->g.N, host, sizeof(double) * (size_t)h->g.N,
-                                    cudaMemcpyHostToDevice), "immobile concentration");
+    return cuda_check(h, copy_on_stream(h, h->d_imm + (size_t)si * h->g.N, host, sizeof(double) * (size_t)h->g.N, cudaMemcpyHostToDevice),
+                      "immobile concentration");
 }
 
 // A species' concentration field (user index s, FP64 [N]): an immobile species takes it as it is; a
@@ -1256,51 +1259,51 @@ static int ade_grid_for(const void* kern, int smem, int num_sms, int threads, in
 
 template <typename TS, typename TC, bool ODD>
 static void launch_ade_t(clb_handle* h) {
-    ++h->launches;  // one transport launch per call
     const int nm = h->n_mobile;
     const int nb = h->S;  // register bucket covers every species (mobile first, then immobile)
     TS* g = (TS*)h->d_g;
     const TC* u = (const TC*)h->d_u;
     int* mt = mob_table(h);
     const SparseView S = view_of(h->ade_sp);
-    const bool ext = h->ap.law2 != CLB_LAW_NONE || h->ap.dis_on || h->ap.gate_on || h->ap.law == CLB_LAW_SYMBOLIC;
     const AdeExtra X = ade_extra(h);
-#define CLB_ADE(NM, EXT)                                                                                          \
-    do {                                                                                                          \
-        if constexpr (sizeof(TS) >= 4 && ade_pipe_minb<TC, NM>() >= 2) {                                           \
-            if (h->ade_pipe) {                                                                                    \
-            auto kern = k_ade_pipe<TS, TC, ODD, NM, EXT>;                                                          \
-            const int sm = 2 * ade_slot_bytes<TC, NM>();                                                           \
-            const int gr = ade_grid_for((const void*)kern, sm, h->num_sms, ADE_THREADS);                           \
-            kern<<<gr, ADE_THREADS, sm, h->stream>>>(g, h->d_imm, h->d_bio, u, S, h->d_neu, h->ap, nm, mt,        \
-                                                     h->ade_west_end, h->ade_east_begin, X);                      \
-            break;                                                                                                \
-            }                                                                                                     \
-        }                                                                                                         \
-        auto kern = k_ade_aa<TS, TC, ODD, NM, EXT>;                                                               \
-        const int sm = ade_slot_bytes<TC, NM>();                                                                  \
-        const int gr = ade_grid_for((const void*)kern, sm, h->num_sms, ADE_THREADS, ODD ? ADE_RESIDENT : ADE_RESIDENT_EVEN); \
-        kern<<<gr, ADE_THREADS, sm, h->stream>>>(g, h->d_imm, h->d_bio, u, S, h->d_neu, h->ap, nm, mt,            \
-                                                 h->ade_west_end, h->ade_east_begin, X);                          \
-    } while (0)
+    auto staged = [&](auto kern, int sm, int resident) {
+        ++h->launches;  // one transport launch per call
+        const int gr = ade_grid_for((const void*)kern, sm, h->num_sms, ADE_THREADS, resident);
+        kern<<<gr, ADE_THREADS, sm, h->stream>>>(g, h->d_imm, h->d_bio, u, S, h->d_neu, h->ap, nm, mt, h->ade_west_end,
+                                                 h->ade_east_begin, X);
+    };
+    // the pipelined form where it was asked for and two slot sets fit; false: not launched
+    auto pipe = [&](auto NM, auto EXT) {
+        constexpr int B = decltype(NM)::value, E = decltype(EXT)::value;
+        if constexpr (sizeof(TS) >= 4 && ade_pipe_minb<TC, B>() >= 2) {
+            if (h->ade_pipe) {
+                staged(k_ade_pipe<TS, TC, ODD, B, E>, 2 * ade_slot_bytes<TC, B>(), ADE_RESIDENT);
+                return true;
+            }
+        }
+        return false;
+    };
+    auto go = [&](auto NM, auto EXT) {
+        constexpr int B = decltype(NM)::value, E = decltype(EXT)::value;
+        if (pipe(NM, EXT)) return;
+        if constexpr (E == 0) launch_ade_stream(h, ODD);
+        else staged(k_ade_aa<TS, TC, ODD, B, E>, ade_slot_bytes<TC, B>(), ODD ? ADE_RESIDENT : ADE_RESIDENT_EVEN);
+    };
     // EXT: 0 the compiled biotic laws alone; 1 with the abiotic block, dissolution and the
     // thermodynamic gate; 2 also the rate-law files (their interpreter's registers and stack stay
     // out of the other instantiations)
+    using std::integral_constant;
     const bool sym = h->ap.law == CLB_LAW_SYMBOLIC || h->ap.law2 == CLB_LAW_SYMBOLIC;
-    if (sym) {
-        if (nb <= 4) CLB_ADE(4, 2);
-        else if (nb <= 8) CLB_ADE(8, 2);
-        else CLB_ADE(16, 2);
-    } else if (ext) {
-        if (nb <= 4) CLB_ADE(4, 1);
-        else if (nb <= 8) CLB_ADE(8, 1);
-        else CLB_ADE(16, 1);
-    } else if (nb <= 1) CLB_ADE(1, 0);
-    else if (nb <= 2) CLB_ADE(2, 0);
-    else if (nb <= 4) CLB_ADE(4, 0);
-    else if (nb <= 8) CLB_ADE(8, 0);
-    else CLB_ADE(16, 0);
-#undef CLB_ADE
+    auto bucket = [&](auto EXT) {
+        if (nb <= 4) go(integral_constant<int, 4>(), EXT);
+        else if (nb <= 8) go(integral_constant<int, 8>(), EXT);
+        else go(integral_constant<int, 16>(), EXT);
+    };
+    if (sym) bucket(integral_constant<int, 2>());
+    else if (!ade_streams(h->ap)) bucket(integral_constant<int, 1>());
+    else if (nb <= 1) go(integral_constant<int, 1>(), integral_constant<int, 0>());
+    else if (nb <= 2) go(integral_constant<int, 2>(), integral_constant<int, 0>());
+    else bucket(integral_constant<int, 0>());
 }
 
 template <typename TS, typename TC>
@@ -1806,7 +1809,7 @@ clb_status ade_density(clb_handle* h, int s, double* host) {
     s = h->u2i[s];
     const size_t N = (size_t)h->g.N;
     if (h->ap.slot[s] < 0)
-        return cuda_check(h, copy_on_stream(h, host, h->d_imm + (size_t)s * N, sizeof(double) * N, cudaMemcpyDeviceToHost), "immobile copy");
+        return cuda_check(h, copy_on_stream(h, host, h->d_imm + (size_t)s * N, sizeof(double) * (size_t)h->g.N, cudaMemcpyDeviceToHost), "immobile copy");
     // the Neumann planes' stored values as the reference holds them after the last stream
     refresh_neumann(h);
     if (!h->d_stage) {
@@ -1836,14 +1839,13 @@ clb_status ade_density(clb_handle* h, int s, double* host) {
 clb_status ade_biomass(clb_handle* h, int m, double* host) {
     if (!h->ade_ready || m < 0 || m >= h->M) return fail(h, CLB_INVALID_ARG, "no such biomass field");
     h->ca_full = true;
-    return cuda_check(h, copy_on_stream(h, host, h->d_bio + (size_t)m * h->g.N, sizeof(double) * h->g.N, cudaMemcpyDeviceToHost), "biomass copy");
+    return cuda_check(h, copy_on_stream(h, host, h->d_bio + (size_t)m * h->g.N, sizeof(double) * (size_t)h->g.N, cudaMemcpyDeviceToHost), "biomass copy");
 }
 
 clb_status ade_set_biomass_field(clb_handle* h, int m, const double* host) {
     if (!h->ade_ready || m < 0 || m >= h->M) return fail(h, CLB_INVALID_ARG, "no such biomass field");
     h->ca_full = true;
-    clb_status st = cuda_check(
-        h, copy_on_stream(h, h->d_bio + (size_t)m * h->g.N, host, sizeof(double) * h->g.N, cudaMemcpyHostToDevice), "biomass copy");
+    clb_status st = cuda_check(h, copy_on_stream(h, h->d_bio + (size_t)m * h->g.N, host, sizeof(double) * (size_t)h->g.N, cudaMemcpyHostToDevice), "biomass copy");
     return st == CLB_OK ? refresh_bflag(h) : st;
 }
 

@@ -391,6 +391,10 @@ clb_status ade_set_thermo(clb_handle* h, const clb_thermo_desc* d);
 clb_status ade_set_immobile(clb_handle* h, int s, const double* host);
 clb_status ade_set_concentration(clb_handle* h, int s, const double* host);
 void ade_refresh_neumann(clb_handle* h);
+// ade_stream.cu: the step with every species streamed through registers, for the laws that allow it
+// (no abiotic law, dissolution, gate or rate-law file)
+bool ade_streams(const AdeParams& P);
+void launch_ade_stream(clb_handle* h, bool odd);
 void ade_free(clb_handle* h);
 
 // geometry_update.cu
