@@ -707,35 +707,82 @@ __global__ void k_ade_get_pops(const TS* __restrict__ g, const TS* __restrict__ 
     }
 }
 
-// computeDensity of species s (internal index) at every voxel: BGK nodes of a Dirichlet / Neumann
-// plane report the stored value; every other voxel 1 + the sum of its incoming populations (a voxel
-// that is not a node holds the initial equilibrium at c0).
+// computeDensity of species s (internal index) at the voxels of rows [r0, r1): BGK nodes of a
+// Dirichlet / Neumann plane report the stored value; every other voxel 1 + the sum of its incoming
+// populations (a voxel that is not a node holds the initial equilibrium at c0). Output: the rows' first
+// voxel at position 0. A stored node's slots come from the step's metadata, a wall's from its six
+// neighbours' compact indices; through the inverse index with 64-bit divisions a species of the 256^3
+// pack took 760 us (FP32), here 211 us (63 us for its bytes; the copy to the host takes 2400 us).
 template <typename TS>
-__global__ void k_ade_density(const TS* __restrict__ g, const TS* __restrict__ glink, const SparseView S,
+__global__ void __launch_bounds__(256) k_ade_density(const TS* __restrict__ g, const TS* __restrict__ glink, const SparseView S,
                               const int8_t* __restrict__ mat, const AdeParams P, int s, int odd,
-                              const double* __restrict__ neu, double* __restrict__ out) {
+                              const double* __restrict__ neu, int r0, int r1, double* __restrict__ out) {
     const Geom G = P.g;
-    double init[7];
-    for (int i = 0; i < 7; ++i) init[i] = q7w(i) * (P.c0[s] - ade_sigma<TS>());
-    for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < G.N; n += (int64_t)gridDim.x * blockDim.x) {
-        const int x = (int)(n / G.plane);
-        const int p = (int)(n - (int64_t)x * G.plane);
+    const int64_t n0 = (int64_t)r0 * G.nz;
+    const double c0 = P.c0[s];
+    const uint32_t K32 = (uint32_t)S.KS;
+    for_each_voxel(G, r0, r1, [&](int64_t n, int x, int y, int z) {
         const int dyn = P.dyn[(uint8_t)mat[n]];
         const bool bgk = dyn == ADE_PORE || dyn == ADE_BIO;
+        const int p = y * G.nz + z;
         if (bgk && x == 0 && P.ltype[s] != CLB_CLOSED) {
-            out[n] = P.ltype[s] == CLB_DIRICHLET ? P.lbc[s] : neu[p];
-            continue;
+            out[n - n0] = P.ltype[s] == CLB_DIRICHLET ? P.lbc[s] : neu[p];
+            return;
         }
         if (bgk && x == G.nx - 1 && P.rtype[s] != CLB_CLOSED) {
-            out[n] = P.rtype[s] == CLB_DIRICHLET ? P.rbc[s] : neu[G.plane + p];
-            continue;
+            out[n - n0] = P.rtype[s] == CLB_DIRICHLET ? P.rbc[s] : neu[G.plane + p];
+            return;
         }
-        double v[7];
-        natural<TS, double, 7>(S, G, g, glink, n, odd, init, v);
+        const int k = S.idx_of[n];
         double r = ade_sigma<TS>();
-        for (int i = 0; i < 7; ++i) r += v[i];
-        out[n] = r;
-    }
+        if (k >= 0) {
+            uint32_t off[7];
+            const uint32_t mt = S.meta[k], wm = mt & 0x7Fu;
+            if (!odd) {
+                const uint32_t lb = 7u * K32 + (uint32_t)(S.tlb[k >> 8] + (int)(mt >> 14));
+#pragma unroll
+                for (int i = 0; i < 7; ++i) {
+                    const int oi = q7opp(i);
+                    off[i] = (i != 0 && ((wm >> oi) & 1u)) ? lb + (uint32_t)__popc(wm & ((1u << oi) - 1u))
+                                                           : (uint32_t)(i * K32) + (uint32_t)k;
+                }
+            } else {
+                const uint32_t blk = wm | ((mt >> 7) & 0x7Fu);
+                int nb[7];
+                odd_sources(S, k, *reinterpret_cast<const int2*>(S.dres + 4 * (int64_t)k), nb);
+                off[0] = (uint32_t)k;
+#pragma unroll
+                for (int i = 1; i < 7; ++i) {
+                    const int oi = q7opp(i);
+                    off[i] = ((blk >> oi) & 1u) ? (uint32_t)(i * K32) + (uint32_t)k
+                                                : (uint32_t)(oi * K32) + (uint32_t)nb[i];
+                }
+            }
+            double v[7];
+#pragma unroll
+            for (int i = 0; i < 7; ++i) v[i] = ldd(g + off[i]);
+#pragma unroll
+            for (int i = 0; i < 7; ++i) r += v[i];
+        } else {
+            // a wall: what its stored neighbours a = n - c_i sent into it
+            int ka[7];
+            ka[0] = -1;
+            ka[1] = x + 1 < G.nx ? S.idx_of[n + G.plane] : -1;
+            ka[4] = x > 0 ? S.idx_of[n - G.plane] : -1;
+            ka[2] = y + 1 < G.ny ? S.idx_of[n + G.nz] : -1;
+            ka[5] = y > 0 ? S.idx_of[n - G.nz] : -1;
+            ka[3] = z + 1 < G.nz ? S.idx_of[n + 1] : -1;
+            ka[6] = z > 0 ? S.idx_of[n - 1] : -1;
+#pragma unroll
+            for (int i = 0; i < 7; ++i) {
+                double v = q7w(i) * (c0 - ade_sigma<TS>());
+                if (ka[i] >= 0)
+                    v = ldd(odd ? link_slot(S, glink, ka[i], i) : g + (uint32_t)(q7opp(i) * K32) + (uint32_t)ka[i]);
+                r += v;
+            }
+        }
+        out[n - n0] = r;
+    });
 }
 
 // shifted != 0: `in` holds g_i - t_i; 0: the stored values g_i - sigma t_i
@@ -904,7 +951,6 @@ void ade_free(clb_handle* h) {
     cudaFree(h->d_u); h->d_u = nullptr;
     cudaFree(h->d_neu); h->d_neu = nullptr;
     cudaFree(h->d_red); h->d_red = nullptr;
-    cudaFree(h->d_stage); h->d_stage = nullptr;
     precip_free(h);
     ca_free(h);
     sparse_free(h->ade_sp);
@@ -1812,26 +1858,31 @@ clb_status ade_density(clb_handle* h, int s, double* host) {
         return cuda_check(h, copy_on_stream(h, host, h->d_imm + (size_t)s * N, sizeof(double) * (size_t)h->g.N, cudaMemcpyDeviceToHost), "immobile copy");
     // the Neumann planes' stored values as the reference holds them after the last stream
     refresh_neumann(h);
-    if (!h->d_stage) {
-        cudaError_t e = cudaMalloc(&h->d_stage, sizeof(double) * N);
-        if (e != cudaSuccess) return cuda_check(h, e, "field staging buffer");
-    }
+    int per = 0;
+    const clb_status ss = stage_rows(h, sizeof(double), &per);
+    if (ss != CLB_OK) return ss;
     const int m = h->ap.slot[s];
     const int odd = (int)(h->ade_iters & 1);
     const size_t off = (size_t)m * h->ade_sp.SS;
     const SparseView Sv = view_of(h->ade_sp);
     const double* neu = h->d_neu + (size_t)s * 2 * h->g.plane;
-    const int grid = h->num_sms * 8;
+    const int grid = h->num_sms * 8, rows = h->g.nx * h->g.ny;
+    double* stage = (double*)h->d_stage;
+    cudaError_t e = cudaSuccess;
+    for (int r0 = 0; r0 < rows && e == cudaSuccess; r0 += per) {
+        const int r1 = std::min(rows, r0 + per);
 #define CLB_DENS(TS)                                                                                              \
     k_ade_density<TS><<<grid, 256, 0, h->stream>>>((const TS*)h->d_g + off, (const TS*)h->d_glink + off, Sv, h->d_mat, \
-                                                   h->ap, s, odd, neu, h->d_stage)
-    switch (h->ade_prec) {
-        case CLB_F64: CLB_DENS(double); break;
-        case CLB_F32: CLB_DENS(float); break;
-        default: CLB_DENS(__half); break;
-    }
+                                                   h->ap, s, odd, neu, r0, r1, stage)
+        switch (h->ade_prec) {
+            case CLB_F64: CLB_DENS(double); break;
+            case CLB_F32: CLB_DENS(float); break;
+            default: CLB_DENS(__half); break;
+        }
 #undef CLB_DENS
-    cudaError_t e = cudaMemcpyAsync(host, h->d_stage, sizeof(double) * N, cudaMemcpyDeviceToHost, h->stream);
+        const size_t at = (size_t)r0 * h->g.nz, n = (size_t)(r1 - r0) * h->g.nz;
+        e = cudaMemcpyAsync(host + at, stage, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream);
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     return cuda_check(h, e, "concentration copy");
 }

@@ -26,6 +26,21 @@ clb_status cuda_check(clb_handle* h, cudaError_t e, const char* what) {
     return fail(h, e == cudaErrorMemoryAllocation ? CLB_OUT_OF_MEMORY : CLB_CUDA_ERROR, m);
 }
 
+clb_status stage_rows(clb_handle* h, size_t per_voxel, int* rows) {
+    const size_t row = per_voxel * (size_t)h->g.nz, all = per_voxel * (size_t)h->g.N;
+    const size_t need = std::max(row, std::min(all, STAGE_BYTES));
+    if (h->stage_bytes < need) {
+        cudaFree(h->d_stage);
+        h->d_stage = nullptr;
+        h->stage_bytes = 0;
+        const cudaError_t e = cudaMalloc(&h->d_stage, need);
+        if (e != cudaSuccess) return cuda_check(h, e, "field staging buffer");
+        h->stage_bytes = need;
+    }
+    *rows = (int)std::min<size_t>(h->stage_bytes / row, (size_t)h->g.nx * h->g.ny);
+    return CLB_OK;
+}
+
 // The host copy of the material map follows the device's lazily: a mask pass of the automaton that
 // changes voxels marks it stale, and the readers of h_mat refresh it here first, so the automaton
 // moves no map to the host in iterations where nobody reads it.
@@ -110,6 +125,7 @@ clb_status clb_destroy(clb_handle* h) {
     flow_free(h);
     ade_free(h);
     cudaFree(h->d_mat);
+    cudaFree(h->d_stage);
     cudaFree(h->d_mat_flow);
     cudaFree(h->d_err);
     cudaFree(h->d_spec_stats);

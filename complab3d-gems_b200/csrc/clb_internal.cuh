@@ -270,7 +270,8 @@ struct clb_handle_s {
     void* d_u = nullptr;              // [3][K] advection velocity (arithmetic type)
     double* d_neu = nullptr;          // [S][2][ny*nz] stored boundary densities
     double* d_red = nullptr;          // scratch of clb_reduce (partials, then the result)
-    double* d_stage = nullptr;        // [N] staging of a field read back to the host
+    void* d_stage = nullptr;          // staging of a field read back to the host (stage_rows)
+    size_t stage_bytes = 0;
     clb::AdeParams ap;
     int64_t ade_iters = 0;
     int64_t neu_iter = -1;            // iteration whose stream the Neumann store reflects
@@ -340,6 +341,11 @@ struct clb_handle_s {
 namespace clb {
 // error helpers (api.cu)
 clb_status fail(clb_handle* h, clb_status s, const std::string& msg);
+// The handle's staging buffer of a readback, allocated on first use and kept (a cudaMalloc and cudaFree
+// per call took between 0.5 and 25 ms): at most STAGE_BYTES, or one row where a row is larger. *rows:
+// the rows of the box (nz voxels each) it holds at `per_voxel` bytes a voxel.
+constexpr size_t STAGE_BYTES = (size_t)32 << 20;
+clb_status stage_rows(clb_handle* h, size_t per_voxel, int* rows);
 // brings h_mat up to date with the device map after automaton passes changed it (api.cu)
 clb_status host_mat_sync(clb_handle* h);
 clb_status cuda_check(clb_handle* h, cudaError_t e, const char* what);

@@ -166,6 +166,28 @@ __device__ __forceinline__ uint32_t odd_dst(int i, int64_t k, const OddRows& R, 
     return (uint32_t)(i * K32) + (uint32_t)dst;
 }
 
+// The incoming populations of stored node k before a step of parity `odd`, from the step's own
+// metadata (the slots natural() finds through the inverse index, without its lookups).
+template <typename TS, typename TC>
+__device__ __forceinline__ void flow_incoming(const SparseView& S, const TS* __restrict__ f, const TS* __restrict__ link,
+                                              int64_t k, int odd, TC (&g)[19]) {
+    const uint32_t K32 = (uint32_t)S.KS;
+    if (!odd) {
+        const uint32_t m0 = S.meta[2 * k], wm = m0 & 0x7FFFFu;
+        const int lb = S.tlb[(int)(k >> 8)] + (int)(m0 >> 19);
+#pragma unroll
+        for (int i = 0; i < 19; ++i) {
+            const int oi = q19opp(i);
+            const bool wall = i != 0 && ((wm >> oi) & 1u);
+            g[i] = ld<TS, TC>(wall ? link + lb + __popc(wm & ((1u << oi) - 1u)) : f + (uint32_t)(i * K32) + k);
+        }
+    } else {
+        const OddRows R = odd_rows(S, k, flow_meta<true>(S, k));
+#pragma unroll
+        for (int i = 0; i < 19; ++i) g[i] = ld<TS, TC>(f + odd_src(i, k, R, K32));
+    }
+}
+
 // One node of the AA step (the flow lattice's collide-and-stream at compact index k); returns
 // the node's |u|^2 when it is a BGK node (for the stored average energy), else 0. Shared by the
 // single-domain step and the batched step of many domains.

@@ -140,6 +140,20 @@ __device__ __forceinline__ void natural(const SparseView& S, const Geom& G, cons
     }
 }
 
+// A walk over the voxels of rows [r0, r1) of the box (a row: one (x, y) column along z), one warp to
+// 32 consecutive voxels of a row, so a voxel's coordinates cost one 32-bit division per warp step and
+// neighbouring voxels share cache lines. Calls fn(n, x, y, z).
+template <typename F>
+__device__ __forceinline__ void for_each_voxel(const Geom& G, int r0, int r1, F fn) {
+    const uint32_t W = (uint32_t)(G.nz + 31) / 32u, total = (uint32_t)(r1 - r0) * W;
+    const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
+    for (uint32_t w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < total; w += nwarps) {
+        const int r = r0 + (int)(w / W), z = (int)(w % W) * 32 + (int)(threadIdx.x & 31);
+        if (z >= G.nz) continue;
+        fn((int64_t)r * G.nz + z, r / G.ny, r % G.ny, z);
+    }
+}
+
 // Inverse of natural(): write the natural populations of node n into the storage; populations
 // that no stored node ever reads are dropped.
 template <typename TS, int Q>
