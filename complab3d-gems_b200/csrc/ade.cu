@@ -1401,41 +1401,6 @@ __device__ __forceinline__ int batch_find(const int64_t* off, int n, int64_t t) 
     return lo;
 }
 
-// One transport step of every domain (no abiotic law, no dissolution). Each CTA takes a
-// contiguous run of the tile table (tiles are in domain order) and copies a tile's domain
-// description into shared memory when it differs from the previous tile's; the per-node code is
-// the single-domain step's, its parameters read from that copy.
-template <typename TS, typename TC, bool ODD, int NM>
-__global__ void __launch_bounds__(ADE_THREADS, (ade_minb<TC, NM>() > 6 ? 6 : ade_minb<TC, NM>()))
-    k_ade_batch(const BatchView B) {
-    extern __shared__ __align__(16) unsigned char ade_smem[];
-    __shared__ __align__(16) BatchDomain sd;
-    const AdeFrame<TC> F = ade_frame<TC, NM>(ade_smem, 0);
-    const int tid = threadIdx.x;
-    AdeExtra X;
-    X.iface = nullptr;
-    X.xidx = nullptr;
-    X.xdc = nullptr;
-    X.ng = 0;
-    const int per = (B.nat + gridDim.x - 1) / gridDim.x;
-    const int t0 = blockIdx.x * per, t1 = min(B.nat, t0 + per);
-    int cur = -1;
-    for (int t = t0; t < t1; ++t) {
-        const BatchTile T = B.atiles[t];
-        if (T.d != cur) {
-            __syncthreads();  // every thread is done with the previous domain
-            const uint64_t* src = reinterpret_cast<const uint64_t*>(B.dom + T.d);
-            uint64_t* dst = reinterpret_cast<uint64_t*>(&sd);
-            for (int q = tid; q < (int)(sizeof(BatchDomain) / 8); q += ADE_THREADS) dst[q] = src[q];
-            __syncthreads();
-            cur = T.d;
-        }
-        for (int64_t k = T.first + tid; k < T.first + T.count; k += ADE_THREADS)
-            ade_node<TS, TC, ODD, NM, 0>((TS*)sd.g, sd.imm, sd.bio, (const TC*)sd.u, sd.as, sd.neu, sd.ap, sd.n_mobile,
-                                         sd.mob, sd.akw, sd.ake, X, F, k);
-    }
-}
-
 // the Neumann planes of every domain (as k_ade_neumann): one thread per pixel of a face that some
 // species treats as Neumann; the inner neighbour's storage locations serve all those species
 template <typename TS, typename TC>
@@ -1481,52 +1446,6 @@ void launch_neumann_batch(const BatchView& B, int prec, bool odd, int grid, cuda
         case CLB_F64: k_neumann_batch<double, double><<<grid, 256, 0, st>>>(B, odd ? 1 : 0); break;
         case CLB_F32: k_neumann_batch<float, float><<<grid, 256, 0, st>>>(B, odd ? 1 : 0); break;
         default: k_neumann_batch<__half, float><<<grid, 256, 0, st>>>(B, odd ? 1 : 0); break;
-    }
-}
-
-// `resident` blocks per SM the shared-memory carveout is sized for (the rest of the SM stays L1,
-// which the odd step's neighbour gathers reuse); set on every launch, since the batch's autotuner
-// tries several
-template <typename TS, typename TC, bool ODD, int NM>
-static void launch_ade_batch_t(const BatchView& B, int grid_mult, int resident, int num_sms, cudaStream_t st) {
-    auto kern = k_ade_batch<TS, TC, ODD, NM>;
-    const int sm = ade_slot_bytes<TC, NM>();
-    const int per_block = sm + (int)sizeof(BatchDomain) + 1024;  // the runtime reserves 1 KB per block
-    const int fit = std::max(1, std::min(resident, (228 * 1024) / per_block));
-    const int pct = std::min(100, (int)((100LL * fit * per_block + 228 * 1024 - 1) / (228 * 1024)));
-    if (sm > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
-    int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, ADE_THREADS, sm) != cudaSuccess || nb < 1) nb = 1;
-    nb = std::min(nb, fit);
-    const int grid = std::max(1, std::min(nb * num_sms * grid_mult, B.nat));
-    kern<<<grid, ADE_THREADS, sm, st>>>(B);
-}
-
-template <typename TS, typename TC, bool ODD>
-static void launch_ade_batch_p(const BatchView& B, int nm, int grid_mult, int resident, int num_sms, cudaStream_t st) {
-    if (nm <= 1) launch_ade_batch_t<TS, TC, ODD, 1>(B, grid_mult, resident, num_sms, st);
-    else if (nm <= 2) launch_ade_batch_t<TS, TC, ODD, 2>(B, grid_mult, resident, num_sms, st);
-    else if (nm <= 4) launch_ade_batch_t<TS, TC, ODD, 4>(B, grid_mult, resident, num_sms, st);
-    else if (nm <= 8) launch_ade_batch_t<TS, TC, ODD, 8>(B, grid_mult, resident, num_sms, st);
-    else launch_ade_batch_t<TS, TC, ODD, 16>(B, grid_mult, resident, num_sms, st);
-}
-
-void launch_ade_batch(const BatchView& B, int prec, bool odd, int nm, int grid_mult, int resident, int num_sms,
-                      cudaStream_t st) {
-    switch (prec) {
-        case CLB_F64:
-            if (odd) launch_ade_batch_p<double, double, true>(B, nm, grid_mult, resident, num_sms, st);
-            else launch_ade_batch_p<double, double, false>(B, nm, grid_mult, resident, num_sms, st);
-            break;
-        case CLB_F32:
-            if (odd) launch_ade_batch_p<float, float, true>(B, nm, grid_mult, resident, num_sms, st);
-            else launch_ade_batch_p<float, float, false>(B, nm, grid_mult, resident, num_sms, st);
-            break;
-        default:
-            if (odd) launch_ade_batch_p<__half, float, true>(B, nm, grid_mult, resident, num_sms, st);
-            else launch_ade_batch_p<__half, float, false>(B, nm, grid_mult, resident, num_sms, st);
-            break;
     }
 }
 

@@ -93,6 +93,19 @@ __device__ __forceinline__ TC gather(const TS* p) {
     }
 }
 
+// One domain of a batch as the streamed step sees it (device copy, one per domain).
+template <typename TC>
+struct StreamDomain {
+    void* g;
+    double* imm;
+    double* bio;
+    const void* u;
+    const double* neu;
+    int64_t kw, ke;
+    SparseView S;
+    AdeStep<TC> P;
+};
+
 // The increment of a species from its rate, with the thresholds and the clamp dC = max(R dt, -C).
 template <typename TC>
 __device__ __forceinline__ TC clamped_increment(TC R, TC dt, TC C) {

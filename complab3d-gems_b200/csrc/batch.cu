@@ -27,10 +27,11 @@ struct clb_batch_s {
     int64_t *d_foff = nullptr, *d_aoff = nullptr, *d_joff = nullptr, *d_face_off = nullptr;
     clb::NeumannJob* d_jobs = nullptr;
     clb::BatchTile *d_ftiles = nullptr, *d_atiles = nullptr;
+    void* d_sdom = nullptr;       // StreamDomain of every domain
     clb::NeumannFace* d_faces = nullptr;
     clb::BatchView view{};
     int64_t flow_nodes = 0, ade_nodes = 0;
-    int flow_threads = 256, flow_mult = 4, ade_mult = 1, ade_resident = 4, neu_grid = 148;
+    int flow_threads = 256, flow_mult = 4, neu_grid = 148;
     bool flow_staged = false;  // the flow step through the staged kernels (4- and 8-byte storage)
     // graphs by (flow parity, ade parity, flow, ade, steps per launch (0: per lattice), tile, lag)
     std::map<std::tuple<int, int, int, int, int, int, int>, cudaGraphExec_t> graphs;
@@ -84,6 +85,7 @@ static void batch_free(clb_batch* b) {
     cudaFree(b->d_joff);
     cudaFree(b->d_ftiles);
     cudaFree(b->d_atiles);
+    cudaFree(b->d_sdom);
     cudaFree(b->d_faces);
     cudaFree(b->d_face_off);
     if (b->stream) cudaStreamDestroy(b->stream);
@@ -165,8 +167,6 @@ clb_status batch_create(clb_handle* const* hs, int n, clb_batch** out) {
             d.n_mobile = h->n_mobile;
             aoff[(size_t)i + 1] = aoff[(size_t)i] + h->ade_sp.K;
             b->ka[(size_t)i] = h->ade_sp.K;
-            for (int64_t k = 0; k < h->ade_sp.K; k += BATCH_ADE_TILE)
-                atiles.push_back({i, (int)std::min<int64_t>(BATCH_ADE_TILE, h->ade_sp.K - k), k});
             for (int side = 0; side < 2; ++side) {
                 bool any = false;
                 for (int s = 0; s < h->S; ++s)
@@ -187,9 +187,24 @@ clb_status batch_create(clb_handle* const* hs, int n, clb_batch** out) {
         }
     }
     b->jbeg[(size_t)n] = (int)jobs.size();
+    cudaError_t e = cudaSuccess;
+    int alaw[5] = {0, 0, 0, 0, 0}, max_mobile = 0;
+    if (b->has_ade) {
+        std::vector<int> form;
+        e = stream_domains(hs, n, b->ade_prec, &b->d_sdom, form);
+        for (int q = 0; q < 4; ++q) {
+            for (int i = 0; i < n; ++i) {
+                const int64_t K = hs[i]->ade_sp.K;
+                max_mobile = std::max(max_mobile, hs[i]->n_mobile);
+                for (int64_t k = 0; form[(size_t)i] == q && k < K; k += BATCH_ADE_TILE)
+                    atiles.push_back({i, (int)std::min<int64_t>(BATCH_ADE_TILE, K - k), k});
+            }
+            alaw[q + 1] = (int)atiles.size();
+        }
+    }
     b->flow_nodes = foff.back();
     b->ade_nodes = aoff.back();
-    cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_dom, sizeof(BatchDomain) * n);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_foff, sizeof(int64_t) * (n + 1));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_aoff, sizeof(int64_t) * (n + 1));
@@ -234,7 +249,9 @@ clb_status batch_create(clb_handle* const* hs, int n, clb_batch** out) {
     b->view.ftiles = b->d_ftiles;
     b->view.nft = (int)ftiles.size();
     b->view.atiles = b->d_atiles;
-    b->view.nat = (int)atiles.size();
+    for (int q = 0; q < 5; ++q) b->view.alaw[q] = alaw[q];
+    b->view.sdom = b->d_sdom;
+    b->view.max_mobile = max_mobile;
     b->view.faces = b->d_faces;
     b->view.foff_faces = b->d_face_off;
     b->view.nfaces = (int)faces.size();
@@ -332,7 +349,7 @@ static void batch_launch_step(clb_batch* b, int fodd, int aodd, bool flow, bool 
     }
     if (ade) {
         launch_neumann_batch(b->view, b->ade_prec, aodd != 0, b->neu_grid, bstream(b));
-        launch_ade_batch(b->view, b->ade_prec, aodd != 0, b->nm, b->ade_mult, b->ade_resident, b->num_sms, bstream(b));
+        launch_ade_batch(b->view, b->ade_prec, aodd != 0, bstream(b));
     }
 }
 
@@ -454,9 +471,8 @@ clb_status batch_step(clb_batch* b, int n, int flow_on, int ade_on) {
 }
 
 // Times the schedules of the batched steps and keeps the fastest. Per-lattice launches: flow with
-// 128 or 256 threads per block and 2, 4 or 8 blocks per SM, or the staged flow kernels; transport
-// with shared memory for 4 or 6 resident blocks per SM and 1 or 2 times the resident grid. Persistent launches (when the lattices share one storage type): tiles of 1024,
-// 2048 or 4096 nodes, lags of 2, 8 or 32 domains, 2 or 8 steps per launch, registers budgeted for
+// 128 or 256 threads per block and 2, 4 or 8 blocks per SM, or the staged flow kernels; transport has
+// one form. Persistent launches (when the lattices share one storage type): tiles of 1024, 2048 or 4096 nodes, lags of 2, 8 or 32 domains, 2 or 8 steps per launch, registers budgeted for
 // 4, 6 or 8 resident CTAs per SM where those kernels are built. Every timed step is a
 // real step of the domains: their iteration counters show the advance.
 clb_status batch_autotune(clb_batch* b, int steps, char* report, int report_len) {
@@ -533,21 +549,11 @@ clb_status batch_autotune(clb_batch* b, int steps, char* report, int report_len)
         legacy += best;
     }
     if (b->has_ade) {
-        float best = 1e30f;
-        int bm = 1, br = 4;
-        for (int resident : {4, 6})
-            for (int mult : {1, 2}) {
-                b->ade_mult = mult;
-                b->ade_resident = resident;
-                const float ms = time_steps(false, true);
-                char buf[96];
-                std::snprintf(buf, sizeof buf, "transport %dx%d:%.1fus ", resident, mult, ms * 1e3f);
-                rep += buf;
-                if (ms < best) { best = ms; bm = mult; br = resident; }
-            }
-        b->ade_mult = bm;
-        b->ade_resident = br;
-        legacy += best;
+        const float ms = time_steps(false, true);
+        char buf[96];
+        std::snprintf(buf, sizeof buf, "transport:%.1fus ", ms * 1e3f);
+        rep += buf;
+        legacy += ms;
     }
     // the flow and transport steps of the per-lattice schedule run one after the other
     b->persistent = false;

@@ -41,7 +41,7 @@ struct BatchTile {
     int64_t first;
 };
 constexpr int BATCH_FLOW_TILE = 1024;  // flow nodes per tile
-constexpr int BATCH_ADE_TILE = 512;    // transport nodes per tile
+constexpr int BATCH_ADE_TILE = 512;    // transport nodes per tile (one block; 128 nodes at a time)
 // the staged flow kernels step whole 256-node tiles of the layout: a run of the tile table must not
 // split one
 static_assert(BATCH_FLOW_TILE % TILE == 0, "flow tiles are whole layout tiles");
@@ -61,8 +61,10 @@ struct BatchView {
     int njobs;
     const BatchTile* ftiles;  // flow tiles, domain by domain
     int nft;
-    const BatchTile* atiles;  // transport tiles, domain by domain
-    int nat;
+    const BatchTile* atiles;  // transport tiles, by the streamed form of their domain's law, then domain by domain
+    int alaw[5];              // the tiles of form q are atiles[alaw[q] .. alaw[q + 1])
+    const void* sdom;         // StreamDomain of every domain
+    int max_mobile;
     const NeumannFace* faces;
     const int64_t* foff_faces;  // [nfaces + 1] prefix sums of the face sizes
     int nfaces;
@@ -102,11 +104,14 @@ struct PersistView {
 void launch_flow_batch(const BatchView& B, int prec, bool odd, int grid, int threads, cudaStream_t st);
 bool flow_batch_staged_available(int prec);
 void launch_flow_batch_staged(const BatchView& B, int prec, bool odd, int num_sms, cudaStream_t st);
-// ade.cu (nm: species register bucket 1, 2, 4, 8 or 16)
-void launch_ade_batch(const BatchView& B, int prec, bool odd, int nm, int grid_mult, int resident, int num_sms,
-                      cudaStream_t st);
+// ade_stream.cu: the transport step of every domain; the device copies its tiles refer to (form: the
+// streamed form of each handle's law)
+void launch_ade_batch(const BatchView& B, int prec, bool odd, cudaStream_t st);
+cudaError_t stream_domains(clb_handle* const* hs, int n, int prec, void** dev, std::vector<int>& form);
+// ade.cu
 void launch_neumann_batch(const BatchView& B, int prec, bool odd, int grid, cudaStream_t st);
-// the persistent schedule: one launch runs the whole item table
+// the persistent schedule: one launch runs the whole item table (nm: species register bucket 1, 2, 4,
+// 8 or 16)
 void launch_batch_persistent(const PersistView& V, int prec, int nm, int minb, int blocks_per_sm, int num_sms,
                              cudaStream_t st);
 int batch_persistent_resident(int prec, int nm, int minb);  // resident CTAs per SM of that launch

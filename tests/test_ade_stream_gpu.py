@@ -55,3 +55,24 @@ def test_streamed_step_matches_the_staged_step(clb, shape, prec, law, mobile, im
         D.close()
     for a, b in zip(*out):
         np.testing.assert_allclose(a, b, rtol=TOL[prec], atol=TOL[prec])
+
+
+@pytest.mark.parametrize("prec", ["F64", "F32", "F16S"])
+def test_batch_of_mixed_laws_matches_single_domains(clb, prec):
+    """A batch whose domains hold different laws, species counts and sizes (tiles of every streamed
+    form, ragged ones among them) against the same domains stepped one by one: the same bits."""
+    cases = [(0, 2, 0, 0), (2, 3, 1, 0), (3, 3, 0, 2), (1, 1, 0, 0), (3, 4, 0, 3), (3, 4, 0, 1)]
+    shapes = [(9, 8, 17), (22, 11, 33), (14, 13, 12), (4, 3, 3), (18, 9, 21), (30, 16, 16)]
+    A, B = ([domain(clb, sh, prec, *c, False, 3 + i) for i, (sh, c) in enumerate(zip(shapes, cases))] for _ in range(2))
+    batch = clb.Batch(B)
+    batch.schedule(persistent=False)
+    for n in (7, 2):
+        batch.step(n, flow=False, transport=True)
+        for D in A:
+            D.ade_step(n)
+    for a, b, c in zip(A, B, cases):
+        for s in range(c[1] + c[2]):
+            np.testing.assert_array_equal(a.concentration(s), b.concentration(s))
+        for m in range(c[3]):
+            np.testing.assert_array_equal(a.biomass(m), b.biomass(m))
+    batch.close()
