@@ -175,6 +175,7 @@ clb_status clb_get_stream(clb_handle* h, void** stream) {
 clb_status clb_tune(clb_handle* h, const char* key, int value) {
     if (!h || !key) return fail(h, CLB_INVALID_ARG, "null argument");
     const std::string k = key;
+    if (k.compare(0, 5, "flow_") == 0) h->flow_tuned = true;  // the per-step kernels the key chooses between
     if (k == "flow_even_tma") { h->flow_even_tma = value ? 1 : 0; return CLB_OK; }
     if (k == "ade_pipe") { h->ade_pipe = value ? 1 : 0; return CLB_OK; }
     if (k == "flow_odd_pipe") {

@@ -245,6 +245,9 @@ struct clb_handle_s {
     int flow_minb = 3;                // minimum resident CTAs per SM of the gather/scatter step (2 or 3)
     int flow_even_grid = 0;
     int flow_odd_pipe = 1;            // odd step pipelined through shared memory (4- and 8-byte storage)
+    int flow_multi = 0;               // blocks of the many-step launch of a small lattice; 0: one launch per step
+    bool flow_multi_one = false;      // its threads keep one node each
+    bool flow_tuned = false;          // a per-step kernel variant was asked for (clb_tune) or measured faster
     int flow_pipe_grid = 0;           // its resident-CTA grid; 0 where it is not available
     int* d_err = nullptr;             // device error flag (bounded waits that gave up)
     uint8_t* d_bflag = nullptr;       // [K] species-lattice nodes where biomass may act (AdeParams::bflag)

@@ -28,6 +28,7 @@
 // 16 bytes neighbour-row offsets (odd step).
 #include "batch.cuh"
 #include "flow_node.cuh"
+#include "grid_sync.cuh"
 #include "tma.cuh"
 
 #include <algorithm>
@@ -322,6 +323,162 @@ __global__ void __launch_bounds__(TILE, sizeof(TS) == 8 ? 2 : 4)
     __shared__ double sh[32];
     double bt = block_sum(esum, sh);
     finish_step(tr, partials, bt, P.n_bgk, trace);
+}
+
+// ------------------------------------------------------------------ many steps of a small lattice
+
+// `steps` AA steps in one cooperative launch, for lattices small enough that a step is mostly latency:
+// launch, ramp-up and metadata are paid once, and between steps the blocks meet at a grid-wide barrier.
+// ONE: every node has a resident thread, which keeps its node's slots of both parities in registers
+// (both steps are in-place permutations of 19 slots); otherwise the resident threads walk the nodes
+// with the per-step code. The barrier also carries the blocks' energy sums, which every block adds up
+// in the same order, so each runs the tracer on its own copy of the window and all stop at the same
+// step; the tracer's sums of a step run while the next step's populations are on their way, its
+// decision before that step's first store.
+constexpr int MULTI_THREADS = 256;
+
+template <typename TS, typename TC, int TRACE, bool ONE>
+__global__ void __launch_bounds__(MULTI_THREADS, 2)
+    k_flow_multi(TS* f, TS* link, const SparseView S, const FlowParams P, Tracer* tr, double* partials, GridSync* gs, int steps,
+                 int odd, int64_t k_west_end, int64_t k_east_begin, int* err) {
+    __shared__ double sh[32];
+    __shared__ double ring[TRACE ? TRACER_WINDOW : 1];
+    __shared__ int s_conv;  // the tracer's decision: set once, before the step after the one it settles
+    if (TRACE && tr->converged) return;  // a batch continues past convergence as no-ops
+    const int tid = threadIdx.x;
+    if (tid == 0) s_conv = 0;
+    const int64_t k = (int64_t)blockIdx.x * MULTI_THREADS + tid, stride = (int64_t)gridDim.x * MULTI_THREADS;
+    const uint32_t K32 = (uint32_t)S.KS;
+    bool live = ONE && k < S.K;
+    uint32_t od[19], wm = 0;
+    TS* lk = link;
+    int code = 0;
+    if (live) {
+        const FlowMeta M = flow_meta<true>(S, k);
+        code = M.code;
+        live = P.dyn[code] != DYN_BB;  // a stored bounce-back node: the identity on AA slots
+        const OddRows R = odd_rows(S, k, M);
+#pragma unroll
+        for (int i = 0; i < 19; ++i) od[i] = odd_src(i, k, R, K32);
+        wm = M.m0 & 0x7FFFFu;
+        lk = link + S.tlb[(int)(k >> 8)] + (int)(M.m0 >> 19);
+    }
+    const bool bgk = live && P.dyn[code] == DYN_BGK;
+    const int side = k < k_west_end ? -1 : (k >= k_east_begin ? 1 : 0);
+    const TC rho = (TC)((side < 0 ? P.rho_w : P.rho_e) - 1.0), omega = (TC)P.omega[code];
+    int head = 0, count = 0;
+    if (TRACE) {
+        for (int q = tid; q < TRACER_WINDOW; q += MULTI_THREADS) ring[q] = tr->ring[q];
+        head = tr->head;
+        count = tr->count;
+    }
+    double energy = 0;
+    // the stored average energy of step `n` (1, 2, ...) from the blocks' sums; with TRACE the tracer's
+    // window and its criterion. By warp 0 alone, while the other warps collide.
+    auto warp_total = [](double v) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        return v;
+    };
+    auto trace = [&](int n) {
+        const double* part = partials + (n & 1) * gridDim.x;
+        double v = 0;
+        for (int q = tid; q < (int)gridDim.x; q += 32) v += __ldcg(part + q);
+        v = warp_total(v);
+        energy = P.n_bgk > 0 ? 0.5 * v / (double)P.n_bgk : 0.0;
+        if (!TRACE) return;
+        if (tid == 0) ring[head] = energy;
+        __syncwarp();
+        head = (head + 1) % TRACER_WINDOW;
+        if (count < TRACER_WINDOW) ++count;
+        if (count < TRACER_WINDOW) return;
+        v = 0;
+        for (int q = tid; q < TRACER_WINDOW; q += 32) v += ring[q];
+        const double mean = warp_total(v) / (double)TRACER_WINDOW;
+        v = 0;
+        for (int q = tid; q < TRACER_WINDOW; q += 32) {
+            const double d = ring[q] - mean;
+            v += d * d;
+        }
+        const double r = sqrt(warp_total(v) / (double)(TRACER_WINDOW - 1)) / mean;
+        if (tid == 0 && (isnan(r) || fabs(r) < tr->eps)) s_conv = 1;
+    };
+    int done = 0;
+    bool ok = true;
+    while (done < steps) {
+        const bool odd_step = ((odd + done) & 1) != 0;
+        TC g[19];
+        if (live) {
+            if (odd_step) {
+#pragma unroll
+                for (int i = 0; i < 19; ++i) g[i] = ld<TS, TC>(f + od[i]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 19; ++i) {
+                    const int oi = q19opp(i);
+                    const bool wall = i != 0 && ((wm >> oi) & 1u);
+                    g[i] = ld<TS, TC>(wall ? lk + __popc(wm & ((1u << oi) - 1u)) : f + (uint32_t)(i * K32) + k);
+                }
+            }
+        }
+        if (TRACE && done > 0 && tid < 32) trace(done);
+        double e = 0;
+        if (bgk) {
+            if (side < 0) regularize19<TC>(g, -1, rho);
+            else if (side > 0) regularize19<TC>(g, 1, rho);
+            e = (double)bgk19<TC>(g, omega);
+        }
+        if (TRACE) {
+            __syncthreads();
+            if (s_conv) break;
+        }
+        if (live) {
+            if (odd_step) {
+#pragma unroll
+                for (int i = 0; i < 19; ++i) st<TS, TC>(f + od[q19opp(i)], g[i]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 19; ++i) {
+                    const bool wall = i != 0 && ((wm >> i) & 1u);
+                    st<TS, TC>(wall ? lk + __popc(wm & ((1u << i) - 1u)) : f + (uint32_t)(q19opp(i) * K32) + k, g[i]);
+                }
+            }
+        }
+        if (!ONE) {
+            if (odd_step) {
+                for (int64_t j = k; j < S.K; j += stride)
+                    e += flow_node<TS, TC, true>(f, link, S, P, j, k_west_end, k_east_begin);
+            } else {
+                for (int64_t j = k; j < S.K; j += stride)
+                    e += flow_node<TS, TC, false>(f, link, S, P, j, k_west_end, k_east_begin);
+            }
+        }
+        ++done;
+        if (TRACE || done == steps) {  // without the tracer only the last step's energy is stored
+            const double bt = block_sum(e, sh);
+            if (tid == 0) partials[(done & 1) * gridDim.x + blockIdx.x] = bt;
+        }
+        if (!(ok = grid_barrier(gs, (unsigned)done))) break;
+    }
+    if (!ok) {
+        if (tid == 0) atomicExch(err, 1);
+        return;
+    }
+    if (blockIdx.x != 0) return;
+    __syncthreads();
+    if (tid < 32 && !s_conv) trace(done);
+    __syncthreads();
+    if (TRACE)
+        for (int q = tid; q < TRACER_WINDOW; q += MULTI_THREADS) tr->ring[q] = ring[q];
+    if (tid == 0) {
+        tr->energy = energy;
+        tr->iterations += done;
+        if (TRACE) {
+            tr->head = head;
+            tr->count = count;
+            if (s_conv) tr->converged = 1;
+        }
+    }
 }
 
 // ------------------------------------------------------------------ batched step of many domains
@@ -783,6 +940,25 @@ static int flow_gather_grid(clb_handle* h) {
     }
 }
 
+// Blocks of k_flow_multi for this lattice, 0 where a launch per step is faster; h->flow_multi_one: every
+// node has a resident thread. us per step, one launch per step -> many steps per launch, by nodes:
+//   11 k: FP64 8.8 -> 4.0, FP32 8.2 -> 3.1, FP16 9.2 -> 3.2;   27 k: 8.8 -> 4.2, 8.2 -> 3.2, 9.2 -> 3.3;
+//   91 k (walked): 13.3 -> 9.1, 10.8 -> 7.4, 12.3 -> 8.4;      214 k: 19.4 -> 14.7, 15.0 -> 11.4, 18.1 -> 13.3;
+//   482 k: 35.9 -> 30.6, 22.5 -> 22.7, 27.9 -> 25.5;           1067 k: 81 -> 79, 45 -> 52, 53 -> 51.
+constexpr int64_t MULTI_MAX_NODES = 400000;
+
+template <typename TS, typename TC>
+static int flow_multi_blocks(clb_handle* h) {
+    int one = 0, loop = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&one, k_flow_multi<TS, TC, 1, true>, MULTI_THREADS, 0) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&loop, k_flow_multi<TS, TC, 1, false>, MULTI_THREADS, 0) != cudaSuccess)
+        return 0;
+    const int64_t need = (h->flow_sp.K + MULTI_THREADS - 1) / MULTI_THREADS;
+    h->flow_multi_one = need <= (int64_t)one * h->num_sms;
+    if (need < 1 || h->flow_sp.K > MULTI_MAX_NODES) return 0;
+    return (int)(h->flow_multi_one ? need : (int64_t)loop * h->num_sms);
+}
+
 clb_status flow_init(clb_handle* h, double delta_p) {
     h->resolve_tracer_valid = false;  // a new flow: the in-loop tracer starts empty again
     const clb_domain_desc& d = h->d;
@@ -894,9 +1070,15 @@ clb_status flow_init(clb_handle* h, double delta_p) {
     if ((e = cudaMalloc(&h->d_partials, sizeof(double) * pcap)) != cudaSuccess) return cuda_check(h, e, "partials");
     h->partial_cap = pcap;
     if (!h->d_err) {
-        if ((e = cudaMalloc(&h->d_err, sizeof(int))) != cudaSuccess) return cuda_check(h, e, "error flag");
+        // [0] the error flag; [2], [3] the grid-wide barrier of the many-step launches
+        if ((e = cudaMalloc(&h->d_err, 4 * sizeof(int))) != cudaSuccess) return cuda_check(h, e, "error flag");
     }
-    cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream);
+    cudaMemsetAsync(h->d_err, 0, 4 * sizeof(int), h->stream);
+    switch (h->flow_prec) {
+        case CLB_F64: h->flow_multi = flow_multi_blocks<double, double>(h); break;
+        case CLB_F32: h->flow_multi = flow_multi_blocks<float, float>(h); break;
+        default: h->flow_multi = flow_multi_blocks<__half, float>(h); break;
+    }
 
     const int ig = h->num_sms * 8;
     const SparseView S = view_of(h->flow_sp);
@@ -960,8 +1142,43 @@ static void launch_flow(clb_handle* h, bool odd, int trace) {
 #undef CLB_LAUNCH_B
 }
 
+template <typename TS, typename TC>
+static cudaError_t launch_flow_multi(clb_handle* h, int n, bool trace) {
+    GridSync* gs = (GridSync*)(h->d_err + 2);
+    cudaError_t e = cudaMemsetAsync(gs, 0, sizeof(GridSync), h->stream);
+    if (e != cudaSuccess) return e;
+    TS *f = (TS*)h->d_f, *link = (TS*)h->d_flink;
+    SparseView S = view_of(h->flow_sp);
+    int odd = (int)(h->flow_iters & 1);
+    void* args[] = {&f, &link, &S, &h->fp, &h->d_tracer, &h->d_partials, &gs, &n, &odd, &h->k_west_end, &h->k_east_begin,
+                    &h->d_err};
+    ++h->launches;
+    const void* kern = h->flow_multi_one
+                           ? (trace ? (const void*)k_flow_multi<TS, TC, 1, true> : (const void*)k_flow_multi<TS, TC, 0, true>)
+                           : (trace ? (const void*)k_flow_multi<TS, TC, 1, false> : (const void*)k_flow_multi<TS, TC, 0, false>);
+    return cudaLaunchCooperativeKernel(kern, dim3(h->flow_multi), dim3(MULTI_THREADS), args, 0, h->stream);
+}
+
+// A small lattice takes its steps in launches of up to MULTI_STEPS (k_flow_multi); a call of one or two
+// steps, and every other lattice, a launch per step.
+constexpr int MULTI_STEPS = 1024, MULTI_MIN_STEPS = 3;
+
 clb_status flow_step(clb_handle* h, int n, bool trace, double eps) {
     (void)eps;
+    if (h->flow_multi && !h->flow_tuned && n >= MULTI_MIN_STEPS) {
+        for (int k = 0; k < n; k += MULTI_STEPS) {
+            const int m = std::min(MULTI_STEPS, n - k);
+            cudaError_t e;
+            switch (h->flow_prec) {
+                case CLB_F64: e = launch_flow_multi<double, double>(h, m, trace); break;
+                case CLB_F32: e = launch_flow_multi<float, float>(h, m, trace); break;
+                default: e = launch_flow_multi<__half, float>(h, m, trace); break;
+            }
+            if (e != cudaSuccess) return cuda_check(h, e, "flow steps");
+            h->flow_iters += m;
+        }
+        return CLB_OK;
+    }
     for (int k = 0; k < n; ++k) {
         launch_flow(h, (h->flow_iters & 1) != 0, trace ? 1 : 0);
         h->flow_iters += 1;
@@ -1177,7 +1394,8 @@ clb_status flow_stats(clb_handle* h, double char_length, clb_flow_stats* out) {
     return CLB_OK;
 }
 
-// Times every kernel variant (even step through TMA tiles or not; odd step compiled for 2 or 3
+// Times every kernel variant (the many-step launch where the lattice is small enough for it; a launch
+// per step: even step through TMA tiles or not; odd step compiled for 2 or 3
 // resident CTAs, or pipelined through shared memory) over `steps` steps and keeps the fastest. The lattice state is saved before
 // and restored after, so the run is unchanged. Writes a one-line report into `report`.
 clb_status flow_autotune(clb_handle* h, int steps, char* report, int report_len) {
@@ -1203,6 +1421,25 @@ clb_status flow_autotune(clb_handle* h, int steps, char* report, int report_len)
     float best = 1e30f;
     int best_tma = save_tma, best_minb = save_minb, best_pipe = save_pipe;
     std::string rep;
+    auto timed = [&]() {
+        flow_step(h, 4, false, 0.0);  // warm
+        cudaEventRecord(a, h->stream);
+        flow_step(h, steps, false, 0.0);
+        cudaEventRecord(b, h->stream);
+        cudaEventSynchronize(b);
+        float ms = 0;
+        cudaEventElapsedTime(&ms, a, b);
+        return ms;
+    };
+    float multi = 1e30f;
+    h->flow_tuned = false;
+    if (h->flow_multi && steps >= MULTI_MIN_STEPS) {
+        multi = timed();
+        char buf[64];
+        snprintf(buf, sizeof(buf), "multi:%.1fus", 1e3f * multi / steps);
+        rep += buf;
+    }
+    h->flow_tuned = true;
     for (int tma = 1; tma >= 0; --tma)
         for (int v = 0; v < 3; ++v) {  // odd step: 3 or 2 resident CTAs, or pipelined
             const int minb = v == 1 ? 2 : 3, pipe = v == 2 ? 1 : 0;
@@ -1211,13 +1448,7 @@ clb_status flow_autotune(clb_handle* h, int steps, char* report, int report_len)
             h->flow_minb = minb;
             h->flow_odd_pipe = pipe;
             h->flow_grid = flow_gather_grid(h);
-            flow_step(h, 2, false, 0.0);  // warm
-            cudaEventRecord(a, h->stream);
-            flow_step(h, steps, false, 0.0);
-            cudaEventRecord(b, h->stream);
-            cudaEventSynchronize(b);
-            float ms = 0;
-            cudaEventElapsedTime(&ms, a, b);
+            const float ms = timed();
             char buf[96];
             if (pipe) snprintf(buf, sizeof(buf), "%stma=%d,pipe:%.1fus", rep.empty() ? "" : " ", tma, 1e3f * ms / steps);
             else snprintf(buf, sizeof(buf), "%stma=%d,minb=%d:%.1fus", rep.empty() ? "" : " ", tma, minb, 1e3f * ms / steps);
@@ -1229,6 +1460,7 @@ clb_status flow_autotune(clb_handle* h, int steps, char* report, int report_len)
     h->flow_even_tma = best_tma;
     h->flow_minb = best_minb;
     h->flow_odd_pipe = best_pipe;
+    h->flow_tuned = best < multi;
     h->flow_grid = flow_gather_grid(h);
     cudaMemcpyAsync(h->d_f, sf, fb, cudaMemcpyDeviceToDevice, h->stream);
     cudaMemcpyAsync(h->d_flink, sl, lb, cudaMemcpyDeviceToDevice, h->stream);
@@ -1238,7 +1470,8 @@ clb_status flow_autotune(clb_handle* h, int steps, char* report, int report_len)
     cudaFree(sl);
     h->flow_iters = iters0;
     char buf[64];
-    if (best_pipe) snprintf(buf, sizeof(buf), " -> tma=%d,pipe", best_tma);
+    if (!h->flow_tuned) snprintf(buf, sizeof(buf), " -> multi");
+    else if (best_pipe) snprintf(buf, sizeof(buf), " -> tma=%d,pipe", best_tma);
     else snprintf(buf, sizeof(buf), " -> tma=%d,minb=%d", best_tma, best_minb);
     rep += buf;
     if (report && report_len > 0) {

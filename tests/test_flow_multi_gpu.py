@@ -1,0 +1,46 @@
+"""Many flow steps in one launch (small lattices) against one launch per step: the same populations
+bit for bit, and the solve's tracer stopping at the same iteration. The per-step kernels are what a
+tuning key selects."""
+import numpy as np
+import pytest
+
+from helpers import mixed_geometry
+
+pytestmark = pytest.mark.gpu
+
+
+def domain(clb, shape, prec, per_step):
+    mat = clb.sphere_pack(*shape, 0.5, 2.0, 4.0, 7) if min(shape) > 40 else mixed_geometry(*shape, seed=4)
+    D = clb.Domain(mat, *shape, 0.8, flow_precision=getattr(clb, prec), bio_codes=(3, 4), perm_ratio=(0.3, 0.0))
+    D.flow_init(2e-4)
+    if per_step:
+        D.tune("flow_min_blocks", 3)
+    return D
+
+
+# a few nodes; a ragged last block; the last size of one node per thread and the first of a walk
+# (148 x 2 x 256 threads); several nodes per thread
+@pytest.mark.parametrize("shape", [(4, 3, 3), (19, 12, 23), (66, 50, 50), (70, 54, 54), (80, 90, 70)])
+@pytest.mark.parametrize("prec", ["F64", "F32", "F16S"])
+def test_many_steps_per_launch_match_single_steps(clb, shape, prec):
+    A, B = (domain(clb, shape, prec, per_step) for per_step in (False, True))
+    for n in (3, 8, 1, 4):  # either parity at the start of a launch, single steps in between
+        A.flow_step(n)
+        B.flow_step(n)
+    np.testing.assert_array_equal(A.flow_populations(), B.flow_populations())
+    a, b = A.flow_stats(), B.flow_stats()
+    assert a["iterations"] == b["iterations"] == 16
+    # the same squares added up in another order: N roundings at most
+    np.testing.assert_allclose(a["energy"], b["energy"], rtol=A.N * 2.0 ** -53)
+
+
+@pytest.mark.parametrize("prec", ["F64", "F32"])
+def test_traced_solve_stops_at_the_same_iteration(clb, prec):
+    A, B = (domain(clb, (19, 12, 23), prec, per_step) for per_step in (False, True))
+    ia, ib = A.flow_solve(5000, 1e-3), B.flow_solve(5000, 1e-3)
+    assert ia == ib and ia[1] and ia[0] > 500
+    np.testing.assert_array_equal(A.flow_populations(), B.flow_populations())
+    # a cap inside a launch, and a second solve that starts from the settled state
+    assert A.flow_solve(7, 1e-12, allow_unconverged=True) == B.flow_solve(7, 1e-12, allow_unconverged=True) == (7, False)
+    assert A.flow_solve(5000, 1e-3) == B.flow_solve(5000, 1e-3)
+    np.testing.assert_array_equal(A.flow_populations(), B.flow_populations())
