@@ -950,6 +950,7 @@ void ade_free(clb_handle* h) {
     cudaFree(h->d_bflag); h->d_bflag = nullptr;
     cudaFree(h->d_u); h->d_u = nullptr;
     cudaFree(h->d_neu); h->d_neu = nullptr;
+    cudaFree(h->d_sync); h->d_sync = nullptr;
     cudaFree(h->d_red); h->d_red = nullptr;
     precip_free(h);
     ca_free(h);
@@ -1040,6 +1041,8 @@ clb_status ade_init(clb_handle* h, const clb_species_desc* sp, int S) {
     if ((e = cudaMalloc(&h->d_u, usize(h->ade_prec) * 3 * K1)) != cudaSuccess) return cuda_check(h, e, "velocity");
     if ((e = cudaMalloc(&h->d_neu, sizeof(double) * S * 2 * h->g.plane + sizeof(int) * 16)) != cudaSuccess)
         return cuda_check(h, e, "boundary store");
+    if ((e = cudaMalloc(&h->d_sync, 4 * sizeof(int))) != cudaSuccess) return cuda_check(h, e, "barrier");
+    cudaMemsetAsync(h->d_sync, 0, 4 * sizeof(int), h->stream);
     if (!h->h_flags) {
         // host-mapped flags the transport step sets (read by the host without a copy)
         if ((e = cudaHostAlloc((void**)&h->h_flags, 16, cudaHostAllocMapped)) != cudaSuccess)
@@ -1682,6 +1685,14 @@ clb_status ade_step(clb_handle* h, int n) {
     if (!h->ade_ready) return fail(h, CLB_NOT_INITIALIZED, "clb_ade_init first");
     if (h->M > 0 && h->d_bio == nullptr) return fail(h, CLB_INVALID_ARG, "biomass missing");
     if (ade_nonfinite_check(h) != CLB_OK) return CLB_NONFINITE;
+    if (ade_streams(h->ap) && !h->ade_pipe && h->spec_mode == CLB_SPEC_OFF) {
+        refresh_neumann(h);  // the values of face nodes whose inner neighbour is no fluid node
+        cudaError_t e;
+        if (launch_ade_multi(h, n, e)) {
+            h->ade_iters += n;
+            return cuda_check(h, e, "ade steps");
+        }
+    }
     for (int k = 0; k < n; ++k) {
         const bool odd = (h->ade_iters & 1) != 0;
         if (h->ap.dis_on) {

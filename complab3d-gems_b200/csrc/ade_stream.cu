@@ -12,6 +12,7 @@
 // 253 -> 186, FP16 Monod 172 -> 84.
 #include "ade_stream.cuh"
 #include "batch.cuh"
+#include "grid_sync.cuh"
 
 #include <algorithm>
 #include <vector>
@@ -75,6 +76,174 @@ void launch_ade_stream(clb_handle* h, bool odd) {
         case CLB_F64: if (odd) launch_stream_t<double, double, true>(h); else launch_stream_t<double, double, false>(h); break;
         case CLB_F32: if (odd) launch_stream_t<float, float, true>(h); else launch_stream_t<float, float, false>(h); break;
         default: if (odd) launch_stream_t<__half, float, true>(h); else launch_stream_t<__half, float, false>(h); break;
+    }
+}
+
+// ------------------------------------------------------------------ many steps of a small lattice
+
+// `steps` steps in one cooperative launch, for lattices small enough that a step is mostly latency (two
+// launches, the Neumann planes' and the step's, their ramp-up and the metadata): the resident threads
+// keep (ONE) or walk their nodes, and the blocks meet at a grid-wide barrier between steps.
+//
+// A Neumann face imposes the density its node's inner neighbour has before the step, which the
+// neighbour's own update overwrites. So the thread of such a face node takes the inner neighbour too: the
+// face node first, reading the neighbour's populations, then the neighbour; the neighbour's own thread
+// leaves it out. (nx >= 4, so that no inner node belongs to two faces.)
+constexpr int STREAM_MULTI_THREADS = 256;
+
+template <typename TS, typename TC, int U, int LAW, bool ONE>
+__global__ void __launch_bounds__(STREAM_MULTI_THREADS, 2)
+    k_ade_stream_multi(TS* g, double* imm, double* bio, const TC* u, const SparseView S, const double* neu, const AdeStep<TC> P,
+                       int64_t kw, int64_t ke, int neumann, int steps, int odd, GridSync* gs, int* err) {
+    extern __shared__ __align__(16) unsigned char stream_smem[];
+    constexpr int T = STREAM_MULTI_THREADS;
+    struct Node {
+        StreamNode<TC> A;
+        uint32_t even[7], odd[7];
+    };
+    auto fluid = [&](int k) {
+        const int d = P.dyn[S.code[k]];
+        return d == ADE_PORE || d == ADE_BIO;
+    };
+    // the x-face partner of node k: for a face node its inner neighbour, for a node next to a face the
+    // face node, where a Neumann face couples the two (both fluid); else -1
+    auto partner = [&](int64_t k) {
+        const int n = S.node[k], x = n / P.plane, nx = (int)(P.N / P.plane);
+        const int d = x == 0 ? 1 : x == 1 ? -1 : x == nx - 1 ? -1 : x == nx - 2 ? 1 : 0;
+        if (d == 0 || !((neumann >> (x <= 1 ? 0 : 1)) & 1)) return -1;
+        const int j = S.idx_of[n + (int64_t)d * P.plane];
+        return j >= 0 && fluid((int)k) && fluid(j) ? j : -1;
+    };
+    auto load = [&](int64_t k) {
+        Node N;
+        const uint32_t mt = S.meta[k];
+        N.A = stream_node<TC, LAW>(S, P, u, k);
+        stream_slots<false>(S, k, mt, N.even);
+        stream_slots<true>(S, k, mt, N.odd);
+        return N;
+    };
+    auto step = [&](int64_t k, const Node& N, int64_t kp, const Node& I, bool odd_step) {
+        auto run = [&](const uint32_t(&off)[7], const uint32_t(&in)[7]) {
+            ade_stream_species<TS, TC, U, LAW, T, false>(
+                g, imm, bio, S, P, kw, ke, stream_smem, k, N.A, off, true, [&](int s, bool west) {
+                    if (kp < 0) return neu[((int64_t)s * 2 + (west ? 0 : 1)) * P.plane + S.node[k] % P.plane];
+                    const TS* f = g + (int64_t)s * S.SS;
+                    double r = ade_sigma<TC>();
+#pragma unroll
+                    for (int i = 0; i < 7; ++i) r += (double)ld<TS, TC>(f + in[i]);
+                    return r;
+                });
+            if (kp >= 0)
+                ade_stream_species<TS, TC, U, LAW, T, false>(g, imm, bio, S, P, kw, ke, stream_smem, kp, I.A, in, true,
+                                                             [](int, bool) { return 0.0; });
+        };
+        if (odd_step) run(N.odd, I.odd);
+        else run(N.even, I.even);
+    };
+    const int64_t k0 = (int64_t)blockIdx.x * T + threadIdx.x, stride = (int64_t)gridDim.x * T;
+    Node N = {}, I = {};
+    int64_t kp = -1;
+    bool mine = false;
+    // a node next to a face whose partner exists belongs to the partner's thread
+    auto place = [&](int64_t k) {
+        const bool face = k < kw || k >= ke;
+        kp = partner(k);
+        mine = face || kp < 0;
+        if (!face) kp = -1;
+        if (mine) {
+            N = load(k);
+            if (kp >= 0) I = load(kp);
+        }
+    };
+    if (ONE && k0 < S.K) place(k0);
+    for (int t = 0; t < steps; ++t) {
+        const bool odd_step = ((odd + t) & 1) != 0;
+        if (ONE) {
+            if (mine) step(k0, N, kp, I, odd_step);
+        } else {
+            for (int64_t k = k0; k < S.K; k += stride) {
+                place(k);
+                if (mine) step(k, N, kp, I, odd_step);
+            }
+        }
+        if (!grid_barrier(gs, (unsigned)t + 1)) {
+            if (threadIdx.x == 0) atomicExch(err, 1);
+            return;
+        }
+    }
+}
+
+// Lattices whose steps go many to a launch, by nodes and by nodes x mobile species. us per step, a
+// launch per step -> many steps per launch (FP64; FP32):
+//   one species:     27 k nodes 10.4 -> 3.0; 10.3 -> 2.8    91 k 12.3 -> 6.6; 11.3 -> 6.2    214 k 14.4 -> 9.0; 12.3 -> 8.2
+//                   482 k 18.5 -> 15.4; 14.8 -> 14.0
+//   three (Monod):   27 k 14.4 -> 6.2; 12.9 -> 5.6          214 k 22.6 -> 16.8; 18.0 -> 13.9  482 k 42 -> 45; 24.9 -> 25.1
+//   eight (dual):    27 k 24.7 -> 15.5; 21.0 -> 13.1         91 k 30.8 -> 28.6; 23.8 -> 22.3  214 k 56.3 -> 56.8; 33.8 -> 31.5
+constexpr int64_t STREAM_MULTI_NODES = 400000, STREAM_MULTI_VALUES = 1500000;
+constexpr int STREAM_MULTI_STEPS = 1024, STREAM_MULTI_MIN_STEPS = 3;
+
+template <typename TS, typename TC>
+static bool launch_stream_multi_t(clb_handle* h, int steps, cudaError_t& e) {
+    SparseView S = view_of(h->ade_sp);
+    if (S.K < 1 || S.K > STREAM_MULTI_NODES || S.K * std::max(1, h->n_mobile) > STREAM_MULTI_VALUES) return false;
+    AdeStep<TC> P = ade_step_params<TC>(h->ap, h->n_mobile);
+    const StreamLaw law = stream_law(P, sizeof(TS));
+    const size_t sm = (size_t)stream_bytes<TC>(law, h->n_mobile) * STREAM_MULTI_THREADS;
+    if (sm > 48 * 1024) return false;
+    int neumann = 0;
+    for (int s = 0; s < h->n_mobile; ++s) {
+        if (P.ltype[s] == CLB_NEUMANN) neumann |= 1;
+        if (P.rtype[s] == CLB_NEUMANN) neumann |= 2;
+    }
+    auto go = [&](auto one, auto walk) {
+        const int64_t need = (S.K + STREAM_MULTI_THREADS - 1) / STREAM_MULTI_THREADS;
+        int per1 = 0, perw = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per1, one, STREAM_MULTI_THREADS, sm) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perw, walk, STREAM_MULTI_THREADS, sm) != cudaSuccess)
+            return false;
+        const bool fits = need <= (int64_t)per1 * h->num_sms;
+        const unsigned grid = (unsigned)(fits ? need : (int64_t)perw * h->num_sms);
+        if (grid == 0) return false;
+        TS* g = (TS*)h->d_g;
+        const TC* u = (const TC*)h->d_u;
+        const double* neu = h->d_neu;
+        GridSync* gs = (GridSync*)(h->d_sync);
+        int* err = h->d_sync + 2;
+        int odd = (int)(h->ade_iters & 1);
+        for (int t = 0; t < steps; t += STREAM_MULTI_STEPS, odd ^= STREAM_MULTI_STEPS & 1) {
+            int n = std::min(STREAM_MULTI_STEPS, steps - t);
+            void* args[] = {&g, &h->d_imm, &h->d_bio, &u, &S, &neu, &P, &h->ade_west_end, &h->ade_east_begin, &neumann, &n, &odd,
+                            &gs, &err};
+            if ((e = cudaMemsetAsync(gs, 0, sizeof(GridSync), h->stream)) != cudaSuccess) return true;
+            ++h->launches;
+            e = cudaLaunchCooperativeKernel(fits ? (const void*)one : (const void*)walk, dim3(grid), dim3(STREAM_MULTI_THREADS), args,
+                                            sm, h->stream);
+            if (e != cudaSuccess) return true;
+        }
+        return true;
+    };
+    constexpr int U = stream_width<TC>();
+    const bool single = h->n_mobile == 1;
+    if (law == STREAM_NONE)
+        return single ? go(k_ade_stream_multi<TS, TC, 1, STREAM_NONE, true>, k_ade_stream_multi<TS, TC, 1, STREAM_NONE, false>)
+                      : go(k_ade_stream_multi<TS, TC, U, STREAM_NONE, true>, k_ade_stream_multi<TS, TC, U, STREAM_NONE, false>);
+    if (law == STREAM_SEPARABLE)
+        return single ? go(k_ade_stream_multi<TS, TC, 1, STREAM_SEPARABLE, true>, k_ade_stream_multi<TS, TC, 1, STREAM_SEPARABLE, false>)
+                      : go(k_ade_stream_multi<TS, TC, U, STREAM_SEPARABLE, true>, k_ade_stream_multi<TS, TC, U, STREAM_SEPARABLE, false>);
+    if (law == STREAM_DUAL_AHEAD)
+        return go(k_ade_stream_multi<TS, TC, U, STREAM_DUAL_AHEAD, true>, k_ade_stream_multi<TS, TC, U, STREAM_DUAL_AHEAD, false>);
+    if constexpr (sizeof(TS) >= 4)
+        return go(k_ade_stream_multi<TS, TC, U, STREAM_DUAL_AFTER, true>, k_ade_stream_multi<TS, TC, U, STREAM_DUAL_AFTER, false>);
+    return false;
+}
+
+bool launch_ade_multi(clb_handle* h, int steps, cudaError_t& e) {
+    e = cudaSuccess;
+    if (steps < STREAM_MULTI_MIN_STEPS || h->g.nx < 4 || !h->d_sync) return false;
+    switch (h->ade_prec) {
+        case CLB_F64: return launch_stream_multi_t<double, double>(h, steps, e);
+        case CLB_F32: return launch_stream_multi_t<float, float>(h, steps, e);
+        default: return launch_stream_multi_t<__half, float>(h, steps, e);
     }
 }
 

@@ -209,68 +209,81 @@ constexpr int stream_bytes(StreamLaw law, int n_mobile) {
          : law == STREAM_DUAL_AHEAD ? n_mobile * (int)sizeof(TC) : 0;
 }
 
-// One node per thread of the transport step; every thread of the block calls it, `on` those that
-// have a node. U: species whose gathers are in flight together. smem: stream_bytes() per thread.
+// The 7 storage slots (from a species' base) of node k in the step of parity ODD.
+template <bool ODD>
+__device__ __forceinline__ void stream_slots(const SparseView& S, int64_t k, uint32_t mt, uint32_t (&off)[7]) {
+    const uint32_t K32 = (uint32_t)S.KS;  // row stride; SS < 2^31 is checked when the layout is built
+    const uint32_t wm = mt & 0x7Fu;
+    if (!ODD) {
+        const uint32_t lb = 7u * K32 + (uint32_t)(S.tlb[(int)(k >> 8)] + (int)(mt >> 14));
+#pragma unroll
+        for (int i = 0; i < 7; ++i) {
+            const int oi = q7opp(i);
+            off[i] = (i != 0 && ((wm >> oi) & 1u)) ? lb + (uint32_t)__popc(wm & ((1u << oi) - 1u))
+                                                   : (uint32_t)(i * K32) + (uint32_t)k;
+        }
+    } else {
+        const uint32_t blk = wm | ((mt >> 7) & 0x7Fu);  // wall or outside the box
+        const int2 dv = *reinterpret_cast<const int2*>(S.dres + 4 * k);
+        const int4 tb = *reinterpret_cast<const int4*>(S.tdb + 4 * (int)(k >> 8));
+        int nb[7];  // compact index of the source node a - c_i
+        nb[0] = (int)k;
+        nb[1] = (int)k + tb.x + (int16_t)(dv.x & 0xFFFF);
+        nb[4] = (int)k + tb.y + (int16_t)((uint32_t)dv.x >> 16);
+        nb[2] = (int)k + tb.z + (int16_t)(dv.y & 0xFFFF);
+        nb[5] = (int)k + tb.w + (int16_t)((uint32_t)dv.y >> 16);
+        nb[3] = (int)k + 1;
+        nb[6] = (int)k - 1;
+        off[0] = (uint32_t)k;
+#pragma unroll
+        for (int i = 1; i < 7; ++i) {
+            const int oi = q7opp(i);
+            off[i] = ((blk >> oi) & 1u) ? (uint32_t)(i * K32) + (uint32_t)k : (uint32_t)(oi * K32) + (uint32_t)nb[i];
+        }
+    }
+}
+
+// What the step knows of a node besides its slots.
+template <typename TC>
+struct StreamNode {
+    int code, nd;  // nd (dense index) only where hb
+    TC ux, uy, uz;
+    bool hb;       // biomass may act (dual Monod)
+};
+
+template <typename TC, int LAW>
+__device__ __forceinline__ StreamNode<TC> stream_node(const SparseView& S, const AdeStep<TC>& P, const TC* __restrict__ u,
+                                                      int64_t k) {
+    StreamNode<TC> A;
+    A.code = S.code[k];
+    A.hb = LAW >= STREAM_DUAL_AFTER && (!P.bflag || P.bflag[k]);
+    A.ux = u[k];
+    A.uy = u[S.K + k];
+    A.uz = u[2 * S.K + k];
+    A.nd = A.hb ? S.node[k] : 0;
+    return A;
+}
+
+// All species of one node, from its slots; every thread of the block calls it, `on` those that have a
+// node. U: species whose gathers are in flight together. smem: stream_bytes() per thread.
+// face(s, west): the density a Neumann face of species s imposes on the node.
 //
-// The barrier before each group keeps the block's warps on the same U species: a step reads and
-// writes 7 rows per species, and warps that drift apart spread their requests over all 7 S rows.
-template <typename TS, typename TC, bool ODD, int U, int LAW, int T>
-__device__ __forceinline__ void ade_stream_node(TS* __restrict__ g, double* __restrict__ imm, double* __restrict__ bio,
-                                                const TC* __restrict__ u, const SparseView& S,
-                                                const double* __restrict__ neu, const AdeStep<TC>& P, int64_t kw,
-                                                int64_t ke, unsigned char* smem, int64_t k, bool on) {
+// LOCKSTEP: the barrier before each group keeps the block's warps on the same U species: a step reads
+// and writes 7 rows per species, and warps that drift apart spread their requests over all 7 S rows.
+template <typename TS, typename TC, int U, int LAW, int T, bool LOCKSTEP, typename Face>
+__device__ __forceinline__ void ade_stream_species(TS* g, double* imm, double* bio, const SparseView& S, const AdeStep<TC>& P,
+                                                   int64_t kw, int64_t ke, unsigned char* smem, int64_t k,
+                                                   const StreamNode<TC>& A, const uint32_t (&off)[7], bool on, Face face_value) {
     double* bs = reinterpret_cast<double*>(smem) + threadIdx.x;  // "after": [STREAM_MICROBES], stride T
     TC* dc = reinterpret_cast<TC*>(smem + (LAW == STREAM_DUAL_AFTER ? STREAM_MICROBES * sizeof(double) * T : 0)) + threadIdx.x;
-    int code = 0, nd = 0;
-    TC ux = 0, uy = 0, uz = 0;
-    uint32_t off[7] = {0, 0, 0, 0, 0, 0, 0};
-    bool hb = false;
-    if (on) {
-        code = S.code[k];
-        const uint32_t mt = S.meta[k];
-        if (LAW >= STREAM_DUAL_AFTER) hb = !P.bflag || P.bflag[k];
-        ux = u[k];
-        uy = u[S.K + k];
-        uz = u[2 * S.K + k];
-        const uint32_t K32 = (uint32_t)S.KS;  // row stride; SS < 2^31 is checked when the layout is built
-        const uint32_t wm = mt & 0x7Fu;
-        if (!ODD) {
-            const uint32_t lb = 7u * K32 + (uint32_t)(S.tlb[(int)(k >> 8)] + (int)(mt >> 14));
-#pragma unroll
-            for (int i = 0; i < 7; ++i) {
-                const int oi = q7opp(i);
-                off[i] = (i != 0 && ((wm >> oi) & 1u)) ? lb + (uint32_t)__popc(wm & ((1u << oi) - 1u))
-                                                       : (uint32_t)(i * K32) + (uint32_t)k;
-            }
-        } else {
-            const uint32_t blk = wm | ((mt >> 7) & 0x7Fu);  // wall or outside the box
-            const int2 dv = *reinterpret_cast<const int2*>(S.dres + 4 * k);
-            const int4 tb = *reinterpret_cast<const int4*>(S.tdb + 4 * (int)(k >> 8));
-            int nb[7];  // compact index of the source node a - c_i
-            nb[0] = (int)k;
-            nb[1] = (int)k + tb.x + (int16_t)(dv.x & 0xFFFF);
-            nb[4] = (int)k + tb.y + (int16_t)((uint32_t)dv.x >> 16);
-            nb[2] = (int)k + tb.z + (int16_t)(dv.y & 0xFFFF);
-            nb[5] = (int)k + tb.w + (int16_t)((uint32_t)dv.y >> 16);
-            nb[3] = (int)k + 1;
-            nb[6] = (int)k - 1;
-            off[0] = (uint32_t)k;
-#pragma unroll
-            for (int i = 1; i < 7; ++i) {
-                const int oi = q7opp(i);
-                off[i] = ((blk >> oi) & 1u) ? (uint32_t)(i * K32) + (uint32_t)k
-                                            : (uint32_t)(oi * K32) + (uint32_t)nb[i];
-            }
-        }
-        if (hb) nd = S.node[k];
-    }
-    const int dyn = P.dyn[code];
+    const int nd = A.nd;
+    const int dyn = P.dyn[A.code];
     on = on && dyn != ADE_BB;  // a voxel sealed by precipitation: the identity on AA slots
     const int nm = P.n_mobile;
     const TC* wk = P.w[dyn == ADE_BIO ? 1 : 0];
     const bool west = k < kw, face = west || k >= ke;
-    const bool react = LAW != STREAM_NONE && on && !face && P.react[code];
-    hb = hb && react;
+    const bool react = LAW != STREAM_NONE && on && !face && P.react[A.code];
+    const bool hb = A.hb && react;
     if (LAW == STREAM_DUAL_AFTER && hb) {
 #pragma unroll
         for (int m = 0; m < STREAM_MICROBES; ++m)
@@ -278,7 +291,7 @@ __device__ __forceinline__ void ade_stream_node(TS* __restrict__ g, double* __re
     }
     TC chk = 0;  // a NaN or infinite density in any species makes the sum non-finite
     for (int s0 = 0; s0 < nm; s0 += U) {
-        if (s0 > 0) __syncthreads();
+        if (LOCKSTEP && s0 > 0) __syncthreads();
         if (!on) continue;
         TC q[U][7];
 #pragma unroll
@@ -317,7 +330,7 @@ __device__ __forceinline__ void ade_stream_node(TS* __restrict__ g, double* __re
                 if (type == CLB_CLOSED) continue;
                 double rs;
                 if (type == CLB_DIRICHLET) rs = west ? P.lbc[s] : P.rbc[s];
-                else rs = neu[((int64_t)s * 2 + (west ? 0 : 1)) * P.plane + S.node[k] % P.plane];
+                else rs = face_value(s, west);
                 TC sum = 0;
 #pragma unroll
                 for (int i = 0; i < 7; ++i)
@@ -342,7 +355,7 @@ __device__ __forceinline__ void ade_stream_node(TS* __restrict__ g, double* __re
                 for (int m = 0; m < STREAM_MICROBES; ++m)
                     if (m < P.M && s == P.acceptor[m]) dc[(1 + m) * T] = r;
             }
-            ade_collide_store<TS, TC>(g + (int64_t)s * S.SS, off, q[v], r, wk[s], d, ux, uy, uz, P.S == 1);
+            ade_collide_store<TS, TC>(g + (int64_t)s * S.SS, off, q[v], r, wk[s], d, A.ux, A.uy, A.uz, P.S == 1);
         }
     }
     if (LAW == STREAM_DUAL_AFTER && hb) {
@@ -374,6 +387,24 @@ __device__ __forceinline__ void ade_stream_node(TS* __restrict__ g, double* __re
             if (d != (TC)0) *c += (double)d;
         }
     if (!isfinite(chk) && P.nonfinite) *(volatile int*)P.nonfinite = 1;
+}
+
+// One node per thread of one transport step; every thread of the block calls it.
+template <typename TS, typename TC, bool ODD, int U, int LAW, int T>
+__device__ __forceinline__ void ade_stream_node(TS* __restrict__ g, double* __restrict__ imm, double* __restrict__ bio,
+                                                const TC* __restrict__ u, const SparseView& S,
+                                                const double* __restrict__ neu, const AdeStep<TC>& P, int64_t kw,
+                                                int64_t ke, unsigned char* smem, int64_t k, bool on) {
+    StreamNode<TC> A = {};
+    uint32_t off[7] = {0, 0, 0, 0, 0, 0, 0};
+    if (on) {
+        const uint32_t mt = S.meta[k];
+        A = stream_node<TC, LAW>(S, P, u, k);
+        stream_slots<ODD>(S, k, mt, off);
+    }
+    ade_stream_species<TS, TC, U, LAW, T, true>(g, imm, bio, S, P, kw, ke, smem, k, A, off, on, [&](int s, bool west) {
+        return neu[((int64_t)s * 2 + (west ? 0 : 1)) * P.plane + S.node[k] % P.plane];
+    });
 }
 
 }  // namespace clb

@@ -147,10 +147,11 @@ clb_status clb_synchronize(clb_handle* h) {
     CLB_ON_DEVICE(h);
     clb_status s = cuda_check(h, cudaStreamSynchronize(h->stream), "synchronize");
     if (s != CLB_OK) return s;
-    if (!h->d_err) return ade_nonfinite_check(h);
-    int flag = 0;
-    copy_on_stream(h, &flag, h->d_err, sizeof(int), cudaMemcpyDeviceToHost);
-    if (flag) return fail(h, CLB_TIMEOUT, "a bounded device wait gave up (bulk copy did not complete)");
+    int flag = 0, flag2 = 0;
+    if (h->d_err) copy_on_stream(h, &flag, h->d_err, sizeof(int), cudaMemcpyDeviceToHost);
+    if (h->d_sync) copy_on_stream(h, &flag2, h->d_sync + 2, sizeof(int), cudaMemcpyDeviceToHost);
+    if (flag || flag2)
+        return fail(h, CLB_TIMEOUT, "a bounded device wait gave up (a bulk copy or a grid-wide barrier did not complete)");
     return ade_nonfinite_check(h);
 }
 

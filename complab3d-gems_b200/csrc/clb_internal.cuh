@@ -271,6 +271,7 @@ struct clb_handle_s {
     double* d_imm = nullptr;          // [S][N] immobile concentrations (unused rows stay empty)
     double* d_bio = nullptr;          // [M][N] biomass
     void* d_u = nullptr;              // [3][K] advection velocity (arithmetic type)
+    int* d_sync = nullptr;            // [0], [1] grid-wide barrier of the many-step launches, [2] its wait gave up
     double* d_neu = nullptr;          // [S][2][ny*nz] stored boundary densities
     double* d_red = nullptr;          // scratch of clb_reduce (partials, then the result)
     void* d_stage = nullptr;          // staging of a field read back to the host (stage_rows)
@@ -404,6 +405,8 @@ void ade_refresh_neumann(clb_handle* h);
 // (no abiotic law, dissolution, gate or rate-law file)
 bool ade_streams(const AdeParams& P);
 void launch_ade_stream(clb_handle* h, bool odd);
+// all of `steps` steps in cooperative launches, where the lattice is small enough; false: not taken
+bool launch_ade_multi(clb_handle* h, int steps, cudaError_t& e);
 void ade_free(clb_handle* h);
 
 // geometry_update.cu

@@ -76,3 +76,21 @@ def test_batch_of_mixed_laws_matches_single_domains(clb, prec):
         for m in range(c[3]):
             np.testing.assert_array_equal(a.biomass(m), b.biomass(m))
     batch.close()
+
+
+@pytest.mark.parametrize("shape", [(3, 5, 6), (4, 3, 3), (9, 8, 17), (66, 50, 50), (70, 54, 54)])
+@pytest.mark.parametrize("prec,law,mobile,immobile,microbes", CASES[:-2])
+def test_many_steps_per_launch_match_single_steps(clb, shape, prec, law, mobile, immobile, microbes):
+    """Steps taken many to a launch (a few nodes, ragged blocks, one node per thread, several) against
+    the same steps launched one by one: the same bits, from either parity."""
+    A, B = (domain(clb, shape, prec, law, mobile, immobile, microbes, False, 5 + mobile) for _ in range(2))
+    for n in (4, 3, 1, 8):
+        A.ade_step(n)
+        for _ in range(n):
+            B.ade_step(1)
+    for s in range(mobile + immobile):
+        np.testing.assert_array_equal(A.concentration(s), B.concentration(s))
+    for m in range(microbes):
+        np.testing.assert_array_equal(A.biomass(m), B.biomass(m))
+    A.close()
+    B.close()
