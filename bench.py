@@ -90,9 +90,13 @@ def replica_throughput(n_open, steps, ms_max, world):
 
 
 def step_kernels(tuned, precision):
-    """Names of the two AA-step kernels the flow step ran (the autotuner's choice, else the
-    library's defaults: tiled even step, pipelined odd step for 4- and 8-byte storage)."""
-    choice = tuned.split("->")[-1] if "->" in tuned else ("tma=1,pipe" if precision != "f16s" else "tma=1,minb=3")
+    """Names of the two AA-step kernels the flow step ran (the autotuner's choice, else the library's
+    default)."""
+    choice = tuned.split("->")[-1] if "->" in tuned else "stream"
+    if "multi" in choice:
+        return "k_flow_multi (many AA steps per launch, mean per step)"
+    if "stream" in choice:
+        return "k_flow_stream (AA even/odd steps, mean per launch)"
     even = "k_flow_even_tma" if "tma=1" in choice else "k_flow_aa<even>"
     odd = "k_flow_odd_pipe" if "pipe" in choice else "k_flow_aa<odd>"
     return f"{even} + {odd} (AA even/odd steps, mean per launch)"

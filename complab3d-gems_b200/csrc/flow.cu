@@ -58,29 +58,17 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
     return r;
 }
 
-// The last block of a step turns the partial sums into the stored average energy and runs
-// the tracer. Deterministic: fixed grid, fixed reduction order.
-__device__ void finish_step(Tracer* tr, double* partials, double block_total, int64_t n_bgk, int trace) {
-    __shared__ bool s_last;
+// The stored average energy of a step from its sum of |u|^2, `count` iterations, and the tracer: by every
+// thread of the step's last block.
+__device__ void settle_step(Tracer* tr, double tot, int64_t n_bgk, int trace, int count) {
     __shared__ double sh[32];
-    if (threadIdx.x == 0) {
-        partials[blockIdx.x] = block_total;
-        __threadfence();
-        unsigned t = atomicAdd(&tr->done_blocks, 1u);
-        s_last = (t == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    double v = 0;
-    for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) v += ((volatile double*)partials)[k];
-    double tot = block_sum(v, sh);
+    double v;
     __shared__ double s_mean;
     __shared__ int s_count;
     if (threadIdx.x == 0) {
         double e = n_bgk > 0 ? 0.5 * tot / (double)n_bgk : 0.0;
         tr->energy = e;
-        tr->iterations += 1;
+        tr->iterations += count;
         tr->done_blocks = 0;
         s_count = 0;
         if (trace) {
@@ -110,7 +98,25 @@ __device__ void finish_step(Tracer* tr, double* partials, double block_total, in
     }
 }
 
-
+// The last block of a step turns the partial sums into the stored average energy and runs
+// the tracer. Deterministic: fixed grid, fixed reduction order.
+__device__ void finish_step(Tracer* tr, double* partials, double block_total, int64_t n_bgk, int trace, int count = 1) {
+    __shared__ bool s_last;
+    __shared__ double sh[32];
+    if (threadIdx.x == 0) {
+        partials[blockIdx.x] = block_total;
+        __threadfence();
+        unsigned t = atomicAdd(&tr->done_blocks, 1u);
+        s_last = (t == gridDim.x - 1);
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    double v = 0;
+    for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) v += ((volatile double*)partials)[k];
+    double tot = block_sum(v, sh);
+    settle_step(tr, tot, n_bgk, trace, count);
+}
 
 // Odd AA step with the gathers of the next node in flight while a node is collided: each thread
 // stages a node's 19 incoming populations in its own two shared-memory slots with asynchronous
@@ -323,6 +329,109 @@ __global__ void __launch_bounds__(TILE, sizeof(TS) == 8 ? 2 : 4)
     __shared__ double sh[32];
     double bt = block_sum(esum, sh);
     finish_step(tr, partials, bt, P.n_bgk, trace);
+}
+
+// ------------------------------------------------------------------ one node per thread
+
+constexpr int STREAM_FLOW_THREADS = 128;
+
+// Resident blocks the registers are budgeted for: 64 registers with 4-byte storage (8 blocks run); 5
+// blocks with 8- and 2-byte storage (FP64 83 us per step on 199x143x131, 87 at 6 and 105 at 8 blocks,
+// which spill; FP16 36.7 us, 37.8 and 40.1).
+template <typename TS>
+constexpr int stream_flow_blocks() { return sizeof(TS) == 4 ? 6 : 5; }
+
+// A gather that keeps its place in program order, so a node's gathers are in flight together.
+template <typename TS, typename TC>
+__device__ __forceinline__ TC gather_flow(const TS* p) {
+    if constexpr (sizeof(TS) == 8) {
+        double v;
+        asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+        return (TC)v;
+    } else if constexpr (sizeof(TS) == 4) {
+        float v;
+        asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+        return (TC)v;
+    } else {
+        unsigned short v;
+        asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
+        return (TC)(__half2float(__ushort_as_half(v)) * HALF_INV);
+    }
+}
+
+// The stored average energy of a streamed step from its warps' sums, and the tracer (a launch after the
+// step's: inside it, a barrier, a fence and a counter per 128-node block cost the FP32 256^3 pack 125 us of a
+// 226 us step).
+__global__ void __launch_bounds__(256) k_flow_energy(const double* __restrict__ warp_sums, int64_t n, Tracer* tr, double* partials,
+                                                     int64_t n_bgk, int trace, int count) {
+    if (trace && tr->converged) return;
+    __shared__ double sh[32];
+    double v = 0;
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) v += warp_sums[q];
+    const double bt = block_sum(v, sh);
+    finish_step(tr, partials, bt, n_bgk, trace, count);
+}
+
+// One AA step, one node per thread, no staging: both steps are in-place permutations of 19 slots of one
+// buffer (the lattice's rows, then its link slots), so a node is 19 offsets, 19 gathers in flight
+// together, the collision and 19 stores. Blocks of 128 nodes in launch order keep the blocks in flight
+// next to one another in every row. ENERGY: the step's stored average energy is wanted (by the tracer
+// after every step, else after the last one of a call): the warps' sums of |u|^2 go to warp_sums.
+//
+// Bound by HBM and the two round trips of a node (metadata, then the gathers). Against the tiled even and
+// the pipelined odd step, us per step: 256x128x128 pack (1.5 M nodes) FP32 60.5 -> 52.4; 384x256x256
+// (8.7 M) FP32 316 -> 292 (4.2 -> 4.6 TB/s of algorithmic traffic); 199x143x131 (1.4 M) FP64 103 -> 83 (5.3
+// TB/s), FP16 71 -> 37. Two to sixteen nodes per thread with the next one's metadata prefetched: 54 to 65
+// us instead of 52.4.
+template <typename TS, typename TC, bool ODD, bool ENERGY>
+__global__ void __launch_bounds__(STREAM_FLOW_THREADS, (stream_flow_blocks<TS>()))
+    k_flow_stream(TS* __restrict__ f, uint32_t link0, const SparseView S, const FlowParams P,
+                  const Tracer* __restrict__ tr, double* __restrict__ warp_sums, int trace, int64_t k_west_end,
+                  int64_t k_east_begin) {
+    // a batch continues past convergence as no-ops: looked at before the stores only, so the load is not a
+    // round trip of its own
+    const int settled = ENERGY && trace ? tr->converged : 0;
+    const int64_t k = (int64_t)blockIdx.x * STREAM_FLOW_THREADS + threadIdx.x;
+    const uint32_t K32 = (uint32_t)S.KS;
+    double e = 0;
+    if (k < S.K) {
+        const FlowMeta M = flow_meta<ODD>(S, k);
+        uint32_t off[19];
+        if (ODD) {
+            const OddRows R = odd_rows(S, k, M);
+#pragma unroll
+            for (int i = 0; i < 19; ++i) off[i] = odd_src(i, k, R, K32);
+        } else {
+            const uint32_t wm = M.m0 & 0x7FFFFu;
+            const uint32_t lb = link0 + (uint32_t)(S.tlb[(int)(k >> 8)] + (int)(M.m0 >> 19));
+#pragma unroll
+            for (int i = 0; i < 19; ++i) {
+                const int oi = q19opp(i);
+                off[i] = (i != 0 && ((wm >> oi) & 1u)) ? lb + (uint32_t)__popc(wm & ((1u << oi) - 1u))
+                                                       : (uint32_t)(i * K32) + (uint32_t)k;
+            }
+        }
+        const int dyn = P.dyn[M.code];
+        if (dyn != DYN_BB) {
+            TC g[19];
+#pragma unroll
+            for (int i = 0; i < 19; ++i) g[i] = gather_flow<TS, TC>(f + off[i]);
+            if (dyn == DYN_BGK) {
+                if (k < k_west_end) regularize19<TC>(g, -1, (TC)(P.rho_w - 1.0));
+                else if (k >= k_east_begin) regularize19<TC>(g, 1, (TC)(P.rho_e - 1.0));
+                e = (double)bgk19<TC>(g, (TC)P.omega[M.code]);
+            }
+            if (!settled) {
+#pragma unroll
+                for (int i = 0; i < 19; ++i) st<TS, TC>(f + off[q19opp(i)], g[i]);
+            }
+        }
+    }
+    if (ENERGY) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
+        if ((threadIdx.x & 31) == 0) warp_sums[((int64_t)blockIdx.x * STREAM_FLOW_THREADS + threadIdx.x) >> 5] = e;
+    }
 }
 
 // ------------------------------------------------------------------ many steps of a small lattice
@@ -889,6 +998,8 @@ __global__ void k_flow_vstats(const double* __restrict__ u, const Geom G, double
 
 // ------------------------------------------------------------------ host side
 
+static int64_t flow_tiles(const clb_handle* h) { return (h->flow_sp.K + STREAM_FLOW_THREADS - 1) / STREAM_FLOW_THREADS; }
+
 static size_t storage_size(int prec) { return prec == CLB_F64 ? 8 : (prec == CLB_F32 ? 4 : 2); }
 
 template <typename TS>
@@ -925,7 +1036,7 @@ static int grid_for(clb_handle* h, F kernel, int threads) {
 
 void flow_free(clb_handle* h) {
     cudaFree(h->d_f); h->d_f = nullptr;
-    cudaFree(h->d_flink); h->d_flink = nullptr;
+    h->d_flink = nullptr;  // inside d_f
     sparse_free(h->flow_sp);
     cudaFree(h->d_tracer); h->d_tracer = nullptr;
     cudaFree(h->d_partials); h->d_partials = nullptr;
@@ -1025,11 +1136,11 @@ clb_status flow_init(clb_handle* h, double delta_p) {
     h->flow_prec = d.flow_precision;
     const size_t es = storage_size(h->flow_prec);
     cudaError_t e;
-    if ((e = cudaMalloc(&h->d_f, es * 19 * (size_t)h->flow_sp.KS)) != cudaSuccess)
+    // one buffer: the 19 population rows, then the link slots
+    const size_t rows = es * 19 * (size_t)h->flow_sp.KS;
+    if ((e = cudaMalloc(&h->d_f, rows + es * (size_t)std::max<int64_t>(1, h->flow_sp.L) + 16)) != cudaSuccess)
         return cuda_check(h, e, "flow populations");
-    // +16 bytes: the FP16 even step copies whole aligned 4-byte words around each link slot
-    if ((e = cudaMalloc(&h->d_flink, es * (size_t)std::max<int64_t>(1, h->flow_sp.L) + 16)) != cudaSuccess)
-        return cuda_check(h, e, "flow links");
+    h->d_flink = (char*)h->d_f + rows;
     if ((e = cudaMalloc(&h->d_tracer, sizeof(Tracer))) != cudaSuccess) return cuda_check(h, e, "tracer");
     cudaMemsetAsync(h->d_tracer, 0, sizeof(Tracer), h->stream);
     cudaMemsetAsync(h->d_flink, 0, es * (size_t)std::max<int64_t>(1, h->flow_sp.L), h->stream);
@@ -1065,9 +1176,10 @@ clb_status flow_init(clb_handle* h, double delta_p) {
         default: h->flow_pipe_grid = 0; break;
     }
     if (!h->flow_pipe_grid) h->flow_odd_pipe = 0;
-    // partials sized for the largest grid any variant uses
+    // the blocks' partials, sized for the largest grid any variant uses, then the streamed step's warp sums
     const int pcap = h->num_sms * 16;
-    if ((e = cudaMalloc(&h->d_partials, sizeof(double) * pcap)) != cudaSuccess) return cuda_check(h, e, "partials");
+    const int64_t warps = std::max<int64_t>(1, flow_tiles(h)) * (STREAM_FLOW_THREADS / 32);
+    if ((e = cudaMalloc(&h->d_partials, sizeof(double) * (pcap + warps))) != cudaSuccess) return cuda_check(h, e, "partials");
     h->partial_cap = pcap;
     if (!h->d_err) {
         // [0] the error flag; [2], [3] the grid-wide barrier of the many-step launches
@@ -1092,11 +1204,45 @@ clb_status flow_init(clb_handle* h, double delta_p) {
     return cuda_check(h, cudaGetLastError(), "flow init");
 }
 
-static void launch_flow(clb_handle* h, bool odd, int trace) {
+// The streamed step, except where a tuning key selects the tiled and pipelined kernels and for a traced FP32
+// step: those form the energy in the step itself, where the streamed one needs a launch after it (482 k
+// nodes FP32 22.3 us per traced step against 24.9, 2.6 M 70 against 73, 6.8 M 251 against 258; FP64 35.1
+// against 34.2, 119 against 111, 455 against 421).
+static bool flow_streams(const clb_handle* h, bool trace) {
+    return !h->flow_tuned && !(trace && h->flow_prec == CLB_F32);
+}
+
+// One step. The streamed step forms the stored energy, and counts `count` iterations, only where count is
+// not 0; the kernels a tuning key selects do both at every step.
+static void launch_flow(clb_handle* h, bool odd, int trace, int count) {
     ++h->launches;  // one step launch per call
     const FlowParams& P = h->fp;
     const SparseView S = view_of(h->flow_sp);
     const int grid = h->flow_grid;
+    if (flow_streams(h, trace)) {
+        const unsigned g = (unsigned)std::max<int64_t>(1, flow_tiles(h));
+        auto go = [&](auto kern, auto* ts) {
+            using TS = std::remove_pointer_t<decltype(ts)>;
+            kern<<<g, STREAM_FLOW_THREADS, 0, h->stream>>>((TS*)h->d_f, (uint32_t)(19 * S.KS), S, P, h->d_tracer,
+                                                           h->d_partials + h->partial_cap, trace, h->k_west_end,
+                                                           h->k_east_begin);
+        };
+#define CLB_STREAM(TS, TC)                                                                                \
+    if (odd) count ? go(k_flow_stream<TS, TC, true, true>, (TS*)nullptr) : go(k_flow_stream<TS, TC, true, false>, (TS*)nullptr); \
+    else count ? go(k_flow_stream<TS, TC, false, true>, (TS*)nullptr) : go(k_flow_stream<TS, TC, false, false>, (TS*)nullptr);
+        switch (h->flow_prec) {
+            case CLB_F64: CLB_STREAM(double, double); break;
+            case CLB_F32: CLB_STREAM(float, float); break;
+            default: CLB_STREAM(__half, float); break;
+        }
+#undef CLB_STREAM
+        if (count) {
+            ++h->launches;
+            k_flow_energy<<<h->num_sms, 256, 0, h->stream>>>(h->d_partials + h->partial_cap, (int64_t)g * (STREAM_FLOW_THREADS / 32),
+                                                             h->d_tracer, h->d_partials, P.n_bgk, trace, count);
+        }
+        return;
+    }
     if (!odd && h->flow_even_tma) {
         const int eg = h->flow_even_grid;
 #define CLB_EVEN(TS, TC)                                                                                       \
@@ -1180,7 +1326,7 @@ clb_status flow_step(clb_handle* h, int n, bool trace, double eps) {
         return CLB_OK;
     }
     for (int k = 0; k < n; ++k) {
-        launch_flow(h, (h->flow_iters & 1) != 0, trace ? 1 : 0);
+        launch_flow(h, (h->flow_iters & 1) != 0, trace ? 1 : 0, trace ? 1 : (k + 1 == n ? n : 0));
         h->flow_iters += 1;
     }
     return cuda_check(h, cudaGetLastError(), "flow step");
@@ -1206,7 +1352,13 @@ clb_status flow_solve(clb_handle* h, int max_it, double eps, int* iterations, bo
     cudaMemcpyAsync(h->d_tracer, &t0, sizeof(Tracer), cudaMemcpyHostToDevice, h->stream);
     const int64_t start = cur.iterations;
     int done = 0;
-    int chunk = 64;
+    // Steps enqueued before the host looks at the tracer. A many-step launch stops itself, so it gets as
+    // many as a launch takes. A streamed step after convergence still reads the lattice (it looks at the
+    // decision before its stores, which saves every other step a round trip), so the run up to a full
+    // window goes at once and then few at a time: the wait costs about 15 us, a step of a lattice that
+    // takes the streamed kernel 16 us and more. The other kernels return at once.
+    const bool multi = h->flow_multi && !h->flow_tuned, stream = !multi && flow_streams(h, true);
+    int chunk = multi ? MULTI_STEPS : stream ? std::max(4, TRACER_WINDOW - t0.count) : 64;
     bool conv = false;
     while (done < max_it) {
         int k = std::min(chunk, max_it - done);
@@ -1217,7 +1369,8 @@ clb_status flow_solve(clb_handle* h, int max_it, double eps, int* iterations, bo
         if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
         if (e != cudaSuccess) return cuda_check(h, e, "tracer read");
         if (cur.converged) { conv = true; break; }
-        if (chunk < 1024) chunk *= 2;
+        if (stream) chunk = chunk >= 32 ? 32 : chunk * 2;
+        else if (chunk < 1024) chunk *= 2;
     }
     h->flow_iters = cur.iterations;  // steps after convergence were no-ops
     if (iterations) *iterations = (int)(cur.iterations - start);
@@ -1394,8 +1547,8 @@ clb_status flow_stats(clb_handle* h, double char_length, clb_flow_stats* out) {
     return CLB_OK;
 }
 
-// Times every kernel variant (the many-step launch where the lattice is small enough for it; a launch
-// per step: even step through TMA tiles or not; odd step compiled for 2 or 3
+// Times every kernel variant (the default: many steps per launch where the lattice is small enough for
+// it, else the streamed step; even step through TMA tiles or not; odd step compiled for 2 or 3
 // resident CTAs, or pipelined through shared memory) over `steps` steps and keeps the fastest. The lattice state is saved before
 // and restored after, so the run is unchanged. Writes a one-line report into `report`.
 clb_status flow_autotune(clb_handle* h, int steps, char* report, int report_len) {
@@ -1431,12 +1584,12 @@ clb_status flow_autotune(clb_handle* h, int steps, char* report, int report_len)
         cudaEventElapsedTime(&ms, a, b);
         return ms;
     };
-    float multi = 1e30f;
     h->flow_tuned = false;
-    if (h->flow_multi && steps >= MULTI_MIN_STEPS) {
-        multi = timed();
+    const float base = timed();
+    const char* base_name = h->flow_multi && steps >= MULTI_MIN_STEPS ? "multi" : "stream";
+    {
         char buf[64];
-        snprintf(buf, sizeof(buf), "multi:%.1fus", 1e3f * multi / steps);
+        snprintf(buf, sizeof(buf), "%s:%.1fus", base_name, 1e3f * base / steps);
         rep += buf;
     }
     h->flow_tuned = true;
@@ -1460,7 +1613,7 @@ clb_status flow_autotune(clb_handle* h, int steps, char* report, int report_len)
     h->flow_even_tma = best_tma;
     h->flow_minb = best_minb;
     h->flow_odd_pipe = best_pipe;
-    h->flow_tuned = best < multi;
+    h->flow_tuned = best < base;
     h->flow_grid = flow_gather_grid(h);
     cudaMemcpyAsync(h->d_f, sf, fb, cudaMemcpyDeviceToDevice, h->stream);
     cudaMemcpyAsync(h->d_flink, sl, lb, cudaMemcpyDeviceToDevice, h->stream);
@@ -1470,7 +1623,7 @@ clb_status flow_autotune(clb_handle* h, int steps, char* report, int report_len)
     cudaFree(sl);
     h->flow_iters = iters0;
     char buf[64];
-    if (!h->flow_tuned) snprintf(buf, sizeof(buf), " -> multi");
+    if (!h->flow_tuned) snprintf(buf, sizeof(buf), " -> %s", base_name);
     else if (best_pipe) snprintf(buf, sizeof(buf), " -> tma=%d,pipe", best_tma);
     else snprintf(buf, sizeof(buf), " -> tma=%d,minb=%d", best_tma, best_minb);
     rep += buf;

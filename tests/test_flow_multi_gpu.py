@@ -44,3 +44,28 @@ def test_traced_solve_stops_at_the_same_iteration(clb, prec):
     assert A.flow_solve(7, 1e-12, allow_unconverged=True) == B.flow_solve(7, 1e-12, allow_unconverged=True) == (7, False)
     assert A.flow_solve(5000, 1e-3) == B.flow_solve(5000, 1e-3)
     np.testing.assert_array_equal(A.flow_populations(), B.flow_populations())
+
+
+@pytest.mark.parametrize("prec", ["F64", "F32", "F16S"])
+def test_streamed_step_matches_the_tiled_step(clb, prec):
+    """A lattice past the many-step limit (the streamed step, plain and traced; a ragged last block)
+    against the tiled and pipelined kernels a tuning key selects: the same bits and iterations."""
+    shape = (90, 101, 110)
+    mat = clb.sphere_pack(*shape, 0.55, 3.0, 6.0, 3)
+    out = []
+    for tuned in (False, True):
+        D = clb.Domain(mat, *shape, 0.8, flow_precision=getattr(clb, prec))
+        D.flow_init(2e-4)
+        if tuned:
+            D.tune("flow_even_tma", 1)
+        D.flow_step(1)
+        D.flow_step(6)
+        stats = D.flow_stats()
+        solved = D.flow_solve(700, 0.2, allow_unconverged=True)
+        out.append((D.flow_populations(), stats, solved, D.flow_stats()["iterations"]))
+        D.close()
+    (fa, sa, va, ia), (fb, sb, vb, ib) = out
+    assert sa["active_nodes"] > 400000 and sa["iterations"] == sb["iterations"] == 7
+    np.testing.assert_allclose(sa["energy"], sb["energy"], rtol=sa["active_nodes"] * 2.0 ** -53)
+    assert va == vb and ia == ib and va[0] >= 500
+    np.testing.assert_array_equal(fa, fb)
