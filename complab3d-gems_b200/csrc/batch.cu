@@ -31,8 +31,8 @@ struct clb_batch_s {
     clb::NeumannFace* d_faces = nullptr;
     clb::BatchView view{};
     int64_t flow_nodes = 0, ade_nodes = 0;
-    int flow_threads = 256, flow_mult = 4, neu_grid = 148;
-    bool flow_staged = false;  // the flow step through the staged kernels (4- and 8-byte storage)
+    int neu_grid = 148;
+    bool flow_staged = false;  // schedule mode 2 was asked for (the same launches as mode 0)
     // graphs by (flow parity, ade parity, flow, ade, steps per launch (0: per lattice), tile, lag)
     std::map<std::tuple<int, int, int, int, int, int, int>, cudaGraphExec_t> graphs;
     // persistent schedule
@@ -255,7 +255,6 @@ clb_status batch_create(clb_handle* const* hs, int n, clb_batch** out) {
     b->view.faces = b->d_faces;
     b->view.foff_faces = b->d_face_off;
     b->view.nfaces = (int)faces.size();
-    b->view.status = b->d_sync;
     b->neu_grid = std::max<int64_t>(1, std::min<int64_t>((face_off.back() + 255) / 256, b->num_sms * 4));
     b->resident = batch_persistent_resident(b->has_ade ? b->ade_prec : b->flow_prec, b->nm, b->minb);
     if (b->has_flow && b->has_ade && b->flow_prec != b->ade_prec) b->persistent = false;  // one storage type per launch
@@ -339,14 +338,7 @@ static clb_status persist_launch(clb_batch* b, int steps, int fodd, int aodd, bo
 
 // one step of the requested lattices at the given parities, on the batch stream
 static void batch_launch_step(clb_batch* b, int fodd, int aodd, bool flow, bool ade) {
-    if (flow) {
-        if (b->flow_staged) {
-            launch_flow_batch_staged(b->view, b->flow_prec, fodd != 0, b->num_sms, bstream(b));
-        } else {
-            const int grid = b->num_sms * b->flow_mult;
-            launch_flow_batch(b->view, b->flow_prec, fodd != 0, grid, b->flow_threads, bstream(b));
-        }
-    }
+    if (flow) launch_flow_batch(b->view, b->flow_prec, fodd != 0, bstream(b));
     if (ade) {
         launch_neumann_batch(b->view, b->ade_prec, aodd != 0, b->neu_grid, bstream(b));
         launch_ade_batch(b->view, b->ade_prec, aodd != 0, bstream(b));
@@ -470,9 +462,9 @@ clb_status batch_step(clb_batch* b, int n, int flow_on, int ade_on) {
     return batch_commit(b, n, flow, ade);
 }
 
-// Times the schedules of the batched steps and keeps the fastest. Per-lattice launches: flow with
-// 128 or 256 threads per block and 2, 4 or 8 blocks per SM, or the staged flow kernels; transport has
-// one form. Persistent launches (when the lattices share one storage type): tiles of 1024, 2048 or 4096 nodes, lags of 2, 8 or 32 domains, 2 or 8 steps per launch, registers budgeted for
+// Times the schedules of the batched steps and keeps the fastest: one launch per lattice and step, or
+// persistent launches (when the lattices share one storage type) with tiles of 1024, 2048 or 4096 nodes,
+// lags of 2, 8 or 32 domains, 2 or 8 steps per launch, registers budgeted for
 // 4, 6 or 8 resident CTAs per SM where those kernels are built. Every timed step is a
 // real step of the domains: their iteration counters show the advance.
 clb_status batch_autotune(clb_batch* b, int steps, char* report, int report_len) {
@@ -521,32 +513,11 @@ clb_status batch_autotune(clb_batch* b, int steps, char* report, int report_len)
     for (clb_handle* h : b->hs) cudaStreamSynchronize(h->stream);
     float legacy = 0.f;
     if (b->has_flow) {
-        float best = 1e30f;
-        int bt = 256, bm = 4;
-        b->flow_staged = false;
-        for (int threads : {128, 256})
-            for (int mult : {2, 4, 8}) {
-                b->flow_threads = threads;
-                b->flow_mult = mult * (256 / threads);
-                const float ms = time_steps(true, false);
-                char buf[96];
-                std::snprintf(buf, sizeof buf, "flow %dx%d:%.1fus ", threads, b->flow_mult, ms * 1e3f);
-                rep += buf;
-                if (ms < best) { best = ms; bt = threads; bm = b->flow_mult; }
-            }
-        bool staged = false;
-        if (flow_batch_staged_available(b->flow_prec)) {
-            b->flow_staged = true;
-            const float ms = time_steps(true, false);
-            char buf[96];
-            std::snprintf(buf, sizeof buf, "flow staged:%.1fus ", ms * 1e3f);
-            rep += buf;
-            if (ms < best) { best = ms; staged = true; }
-        }
-        b->flow_staged = staged;
-        b->flow_threads = bt;
-        b->flow_mult = bm;
-        legacy += best;
+        const float ms = time_steps(true, false);
+        char buf[96];
+        std::snprintf(buf, sizeof buf, "flow:%.1fus ", ms * 1e3f);
+        rep += buf;
+        legacy += ms;
     }
     if (b->has_ade) {
         const float ms = time_steps(false, true);
@@ -640,7 +611,7 @@ clb_status batch_schedule(clb_batch* b, int persistent, int tile, int lag, int s
         b->minb = ctas_per_sm;
         b->resident = batch_persistent_resident(prec, b->nm, ctas_per_sm);
     }
-    if (persistent == 2 && b->has_flow && !flow_batch_staged_available(b->flow_prec))
+    if (persistent == 2 && b->has_flow && b->flow_prec == CLB_F16S)
         return bfail(b, CLB_INVALID_ARG, "schedule: the staged flow step needs 4- or 8-byte flow storage");
     b->persistent = persistent == 1;
     b->flow_staged = persistent == 2;

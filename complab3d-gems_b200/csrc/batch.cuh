@@ -40,12 +40,8 @@ struct BatchTile {
     int count;
     int64_t first;
 };
-constexpr int BATCH_FLOW_TILE = 1024;  // flow nodes per tile
+constexpr int BATCH_FLOW_TILE = 512;   // flow nodes per tile (one block; 128 nodes at a time)
 constexpr int BATCH_ADE_TILE = 512;    // transport nodes per tile (one block; 128 nodes at a time)
-// the staged flow kernels step whole 256-node tiles of the layout: a run of the tile table must not
-// split one
-static_assert(BATCH_FLOW_TILE % TILE == 0, "flow tiles are whole layout tiles");
-
 // One x-face of one domain that at least one mobile species treats as Neumann
 struct NeumannFace {
     int d, side;
@@ -68,7 +64,6 @@ struct BatchView {
     const NeumannFace* faces;
     const int64_t* foff_faces;  // [nfaces + 1] prefix sums of the face sizes
     int nfaces;
-    int* status;  // nonzero: a bounded wait of a staged step gave up
 };
 
 constexpr int BATCH_MAX_DOMAINS = 2048;
@@ -99,11 +94,8 @@ struct PersistView {
     int64_t wait_ns;  // limit of one wait
 };
 
-// flow.cu (staged: the even step through bulk-copied tiles, the odd step with the next node's
-// gathers in flight, 4- and 8-byte storage; else the plain per-node step)
-void launch_flow_batch(const BatchView& B, int prec, bool odd, int grid, int threads, cudaStream_t st);
-bool flow_batch_staged_available(int prec);
-void launch_flow_batch_staged(const BatchView& B, int prec, bool odd, int num_sms, cudaStream_t st);
+// flow.cu
+void launch_flow_batch(const BatchView& B, int prec, bool odd, cudaStream_t st);
 // ade_stream.cu: the transport step of every domain; the device copies its tiles refer to (form: the
 // streamed form of each handle's law)
 void launch_ade_batch(const BatchView& B, int prec, bool odd, cudaStream_t st);
