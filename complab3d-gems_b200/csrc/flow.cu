@@ -598,7 +598,7 @@ __global__ void __launch_bounds__(MULTI_THREADS, 2)
 
 // One AA step of every domain's flow lattice: one block per tile of the table, which takes its domain's
 // flow part to shared memory and steps the tile 128 nodes at a time with the single-domain streamed step's
-// code. 96 uneven domains (2.9 M nodes, FP32): BFLOW us per step; the tiled and pipelined steps over runs of
+// code. 96 uneven domains (2.9 M nodes, FP32): 131 us per step; the tiled and pipelined steps over runs of
 // the table took 145.
 template <typename TS, typename TC, bool ODD>
 __global__ void __launch_bounds__(STREAM_FLOW_THREADS, (stream_flow_blocks<TS>())) k_flow_stream_batch(const BatchView B) {
