@@ -621,53 +621,6 @@ __global__ void __launch_bounds__(ADE_THREADS, (ade_pipe_minb<TC, NM>() < 1 ? 1 
     cp_async_wait_group<0>();
 }
 
-// The stored density of every Neumann plane node: the density of its inner neighbour as it
-// stands before the step (FlatAdiabaticBoundaryFunctional3D after the previous stream). A node
-// whose inner neighbour is not a fluid node keeps its previous value.
-// The Neumann planes of one step, by side (0: x = 0, 1: x = nx - 1): species and mobile slot.
-struct NeumannPlanes {
-    int n[2];
-    int s[2][CLB_MAX_SPECIES], m[2][CLB_MAX_SPECIES];
-};
-
-// One thread per plane pixel and side: the inner neighbour's 7 storage locations are found once
-// (they are the same in every species' buffer, a species stride apart) and serve every species
-// with a Neumann face on that side, whose loads are then all independent.
-template <typename TS, typename TC>
-__global__ void k_ade_neumann(const TS* __restrict__ g, const TS* __restrict__ glink, const SparseView S,
-                              const int8_t* __restrict__ mat, double* __restrict__ neu, const AdeParams P,
-                              const NeumannPlanes J, int odd) {
-    const Geom G = P.g;
-    const int side = blockIdx.y;
-    const int ns = J.n[side];
-    if (ns == 0) return;
-    const int xb = side == 0 ? 0 : G.nx - 1, xi = side == 0 ? 1 : G.nx - 2;
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < G.plane; p += gridDim.x * blockDim.x) {
-        const int64_t nb = (int64_t)xb * G.plane + p, ni = (int64_t)xi * G.plane + p;
-        const int db = P.dyn[mat[nb]], di = P.dyn[mat[ni]];
-        if (!(db == ADE_PORE || db == ADE_BIO) || !(di == ADE_PORE || di == ADE_BIO)) continue;
-        int x, y, z;
-        decode(G, ni, x, y, z);
-        const TS* loc[7];  // in species 0's buffer; nullptr: never written, the initial value
-#pragma unroll
-        for (int i = 0; i < 7; ++i) loc[i] = natural_slot<const TS, 7>(S, G, g, glink, ni, x, y, z, i, odd);
-#pragma unroll 2
-        for (int j = 0; j < ns; ++j) {
-            const int s = J.s[side][j];
-            const int64_t sh = (int64_t)J.m[side][j] * S.SS;
-            const double c0 = P.c0[s];
-            TC pop[7];
-#pragma unroll
-            for (int i = 0; i < 7; ++i)
-                pop[i] = loc[i] ? ld<TS, TC>(loc[i] + sh) : (TC)(q7w(i) * (c0 - ade_sigma<TC>()));
-            double r = ade_sigma<TC>();
-#pragma unroll
-            for (int i = 0; i < 7; ++i) r += (double)pop[i];
-            neu[((int64_t)s * 2 + side) * G.plane + p] = r;
-        }
-    }
-}
-
 template <typename TS>
 __global__ void k_ade_init(TS* __restrict__ g, TS* __restrict__ glink, int64_t K, int64_t L, int64_t SS,
                            int n_mobile, const double* __restrict__ c0m) {
@@ -1355,101 +1308,13 @@ static void launch_ade_t(clb_handle* h) {
     else bucket(integral_constant<int, 0>());
 }
 
-template <typename TS, typename TC>
-static void launch_neumann(clb_handle* h, int odd) {
-    const SparseView S = view_of(h->ade_sp);
-    NeumannPlanes J;
-    J.n[0] = J.n[1] = 0;
-    for (int s = 0; s < h->S; ++s) {
-        const int m = h->ap.slot[s];
-        if (m < 0) continue;
-        for (int side = 0; side < 2; ++side) {
-            const int t = side == 0 ? h->ap.ltype[s] : h->ap.rtype[s];
-            if (t != CLB_NEUMANN) continue;
-            J.s[side][J.n[side]] = s;
-            J.m[side][J.n[side]] = m;
-            ++J.n[side];
-        }
-    }
-    if (J.n[0] + J.n[1] == 0) return;
-    const dim3 grid(std::max(1, std::min(h->num_sms * 4, (h->g.plane + 127) / 128)), 2);
-    ++h->launches;
-    k_ade_neumann<TS, TC><<<grid, 128, 0, h->stream>>>((const TS*)h->d_g, (const TS*)h->d_glink, S, h->d_mat,
-                                                       h->d_neu, h->ap, J, odd);
-}
-
 // The stored densities are those after the latest stream; they are recomputed lazily, once per
 // transport iteration, so that a readback or a change of the material map between two steps
 // (clb_geometry_update refreshes them before it converts voxels) does not alter them.
 static void refresh_neumann(clb_handle* h) {
     if (h->neu_iter == h->ade_iters) return;
     h->neu_iter = h->ade_iters;
-    const int odd = (int)(h->ade_iters & 1);
-    switch (h->ade_prec) {
-        case CLB_F64: launch_neumann<double, double>(h, odd); break;
-        case CLB_F32: launch_neumann<float, float>(h, odd); break;
-        default: launch_neumann<__half, float>(h, odd); break;
-    }
-}
-
-// ------------------------------------------------------------------ batched step of many domains
-
-__device__ __forceinline__ int batch_find(const int64_t* off, int n, int64_t t) {
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (off[mid] <= t) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
-// the Neumann planes of every domain (as k_ade_neumann): one thread per pixel of a face that some
-// species treats as Neumann; the inner neighbour's storage locations serve all those species
-template <typename TS, typename TC>
-__global__ void k_neumann_batch(const BatchView B, int odd) {
-    const int64_t total = B.foff_faces[B.nfaces];
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int j = batch_find(B.foff_faces, B.nfaces, t);
-        const NeumannFace J = B.faces[j];
-        const BatchDomain& d = B.dom[J.d];
-        const Geom G = d.ap.g;
-        const int p = (int)(t - B.foff_faces[j]);
-        const int xb = J.side == 0 ? 0 : G.nx - 1, xi = J.side == 0 ? 1 : G.nx - 2;
-        const int64_t nb = (int64_t)xb * G.plane + p, ni = (int64_t)xi * G.plane + p;
-        const int db = d.ap.dyn[d.mat[nb]], di = d.ap.dyn[d.mat[ni]];
-        if (!(db == ADE_PORE || db == ADE_BIO) || !(di == ADE_PORE || di == ADE_BIO)) continue;
-        int x, y, z;
-        decode(G, ni, x, y, z);
-        const TS* g0 = (const TS*)d.g;
-        const TS* loc[7];
-#pragma unroll
-        for (int i = 0; i < 7; ++i) loc[i] = natural_slot<const TS, 7>(d.as, G, g0, (const TS*)d.glink, ni, x, y, z, i, odd);
-        const int S = d.ap.S;
-        for (int s = 0; s < S; ++s) {
-            const int m = d.ap.slot[s];
-            if (m < 0 || (J.side == 0 ? d.ap.ltype[s] : d.ap.rtype[s]) != CLB_NEUMANN) continue;
-            const int64_t sh = (int64_t)m * d.as.SS;
-            const double c0 = d.ap.c0[s];
-            TC pop[7];
-#pragma unroll
-            for (int i = 0; i < 7; ++i)
-                pop[i] = loc[i] ? ld<TS, TC>(loc[i] + sh) : (TC)(q7w(i) * (c0 - ade_sigma<TC>()));
-            double r = ade_sigma<TC>();
-#pragma unroll
-            for (int i = 0; i < 7; ++i) r += (double)pop[i];
-            d.neu[((int64_t)s * 2 + J.side) * G.plane + p] = r;
-        }
-    }
-}
-
-void launch_neumann_batch(const BatchView& B, int prec, bool odd, int grid, cudaStream_t st) {
-    if (B.nfaces == 0) return;
-    switch (prec) {
-        case CLB_F64: k_neumann_batch<double, double><<<grid, 256, 0, st>>>(B, odd ? 1 : 0); break;
-        case CLB_F32: k_neumann_batch<float, float><<<grid, 256, 0, st>>>(B, odd ? 1 : 0); break;
-        default: k_neumann_batch<__half, float><<<grid, 256, 0, st>>>(B, odd ? 1 : 0); break;
-    }
+    launch_ade_neumann(h, (h->ade_iters & 1) != 0);
 }
 
 // ------------------------------------------------------------------ persistent batched steps
@@ -1499,7 +1364,7 @@ __device__ __forceinline__ TC ld_cg(const TS* p) {
     else return (TC)__ldcg(p);
 }
 
-// k_neumann_batch's value for plane pixel p of job J, with coherent reads
+// The Neumann value (k_neumann, ade_stream.cu) of plane pixel p of job J, with coherent reads
 template <typename TS, typename TC>
 __device__ __forceinline__ void persist_neumann_pixel(const BatchDomain& d, const NeumannJob& J, int p, int odd) {
     const Geom G = d.ap.g;

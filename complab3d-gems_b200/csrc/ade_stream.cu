@@ -79,6 +79,77 @@ void launch_ade_stream(clb_handle* h, bool odd) {
     }
 }
 
+// ------------------------------------------------------------------ Neumann planes
+
+// The stored density of a Neumann plane node is its inner neighbour's as it stands before the step
+// (FlatAdiabaticBoundaryFunctional3D after the previous stream); a node whose inner neighbour is not a
+// fluid node keeps its previous value. One thread per plane pixel, side and species, the neighbour's slots
+// from the step's metadata: three dependent reads (compact indices, metadata, populations), which is what
+// bounds it. FP32, us per step: 8 species of 256x256 pixels 9.1, 96 uneven domains of 3 species 9.8; from
+// the dense neighbour lookups (five dependent reads, 64-bit divisions, a search for the batch's
+// domain) 12.7 and 13.4.
+template <typename TS, typename TC, bool ODD>
+__device__ __forceinline__ void neumann_pixel(const TS* __restrict__ g, const SparseView& S, const int8_t* dyn, int nx, int plane,
+                                              int side, int p, int s, double* __restrict__ neu) {
+    const int64_t nb = side == 0 ? p : (int64_t)(nx - 1) * plane + p, ni = side == 0 ? nb + plane : nb - plane;
+    const int kb = S.idx_of[nb], ki = S.idx_of[ni];
+    if (kb < 0 || ki < 0) return;
+    const int cb = S.code[kb], ci = S.code[ki];
+    uint32_t off[7];
+    stream_slots<ODD>(S, ki, S.meta[ki], off);
+    const int db = dyn[cb], di = dyn[ci];
+    if (!(db == ADE_PORE || db == ADE_BIO) || !(di == ADE_PORE || di == ADE_BIO)) return;
+    const TS* f = g + (int64_t)s * S.SS;
+    TC pop[7];
+#pragma unroll
+    for (int i = 0; i < 7; ++i) pop[i] = ld<TS, TC>(f + off[i]);
+    double r = ade_sigma<TC>();
+#pragma unroll
+    for (int i = 0; i < 7; ++i) r += (double)pop[i];
+    neu[((int64_t)s * 2 + side) * plane + p] = r;
+}
+
+// The species with a Neumann face, by side, and what the planes need of the domain.
+struct NeumannPlanes {
+    int nx, plane;
+    int n[2];
+    int8_t s[2][CLB_MAX_SPECIES];
+    int8_t dyn[MAX_CODES];
+};
+
+template <typename TS, typename TC, bool ODD>
+__global__ void __launch_bounds__(STREAM_THREADS) k_neumann(const TS* __restrict__ g, const SparseView S, const NeumannPlanes J,
+                                                            double* __restrict__ neu) {
+    const int p = blockIdx.x * STREAM_THREADS + threadIdx.x, side = blockIdx.y, j = blockIdx.z;
+    if (p >= J.plane || j >= J.n[side]) return;
+    neumann_pixel<TS, TC, ODD>(g, S, J.dyn, J.nx, J.plane, side, p, J.s[side][j], neu);
+}
+
+void launch_ade_neumann(clb_handle* h, bool odd) {
+    NeumannPlanes J;
+    J.nx = h->g.nx;
+    J.plane = h->g.plane;
+    J.n[0] = J.n[1] = 0;
+    for (int s = 0; s < h->n_mobile; ++s) {  // internal order: the mobile species first
+        if (h->ap.ltype[s] == CLB_NEUMANN) J.s[0][J.n[0]++] = (int8_t)s;
+        if (h->ap.rtype[s] == CLB_NEUMANN) J.s[1][J.n[1]++] = (int8_t)s;
+    }
+    const int most = std::max(J.n[0], J.n[1]);
+    if (most == 0) return;
+    std::memcpy(J.dyn, h->ap.dyn, sizeof(J.dyn));
+    const dim3 grid((unsigned)((h->g.plane + STREAM_THREADS - 1) / STREAM_THREADS), 2, (unsigned)most);
+    ++h->launches;
+#define CLB_NEU(TS, TC)                                                                                                    \
+    if (odd) k_neumann<TS, TC, true><<<grid, STREAM_THREADS, 0, h->stream>>>((const TS*)h->d_g, view_of(h->ade_sp), J, h->d_neu); \
+    else k_neumann<TS, TC, false><<<grid, STREAM_THREADS, 0, h->stream>>>((const TS*)h->d_g, view_of(h->ade_sp), J, h->d_neu);
+    switch (h->ade_prec) {
+        case CLB_F64: CLB_NEU(double, double); break;
+        case CLB_F32: CLB_NEU(float, float); break;
+        default: CLB_NEU(__half, float); break;
+    }
+#undef CLB_NEU
+}
+
 // ------------------------------------------------------------------ many steps of a small lattice
 
 // `steps` steps in one cooperative launch, for lattices small enough that a step is mostly latency (two
@@ -288,6 +359,32 @@ static void launch_stream_batch_t(const BatchView& B, cudaStream_t st) {
     }
     if constexpr (sizeof(TS) >= 4) go(k_ade_stream_batch<TS, TC, ODD, U, STREAM_DUAL_AFTER>, STREAM_DUAL_AFTER);
     go(k_ade_stream_batch<TS, TC, ODD, U, STREAM_DUAL_AHEAD>, STREAM_DUAL_AHEAD);
+}
+
+// the Neumann planes of every domain: one block per run of pixels of a face, one y-block per species
+template <typename TS, typename TC, bool ODD>
+__global__ void __launch_bounds__(STREAM_THREADS) k_neumann_batch(const NeumannTile* __restrict__ tiles,
+                                                                  const StreamDomain<TC>* __restrict__ dom) {
+    const NeumannTile T = tiles[blockIdx.x];
+    const StreamDomain<TC>& D = dom[T.d];
+    const int s = blockIdx.y, p = T.first + (int)threadIdx.x;
+    if (p >= D.P.plane || s >= D.P.n_mobile || (T.side == 0 ? D.P.ltype[s] : D.P.rtype[s]) != CLB_NEUMANN) return;
+    neumann_pixel<TS, TC, ODD>((const TS*)D.g, D.S, D.P.dyn, (int)(D.P.N / D.P.plane), D.P.plane, T.side, p, s,
+                               const_cast<double*>(D.neu));
+}
+
+void launch_neumann_batch(const BatchView& B, int prec, bool odd, cudaStream_t st) {
+    if (B.nnt == 0) return;
+    const dim3 grid((unsigned)B.nnt, (unsigned)std::max(1, B.max_mobile));
+#define CLB_NEU(TS, TC)                                                                                                  \
+    if (odd) k_neumann_batch<TS, TC, true><<<grid, STREAM_THREADS, 0, st>>>(B.ntiles, static_cast<const StreamDomain<TC>*>(B.sdom)); \
+    else k_neumann_batch<TS, TC, false><<<grid, STREAM_THREADS, 0, st>>>(B.ntiles, static_cast<const StreamDomain<TC>*>(B.sdom));
+    switch (prec) {
+        case CLB_F64: CLB_NEU(double, double); break;
+        case CLB_F32: CLB_NEU(float, float); break;
+        default: CLB_NEU(__half, float); break;
+    }
+#undef CLB_NEU
 }
 
 void launch_ade_batch(const BatchView& B, int prec, bool odd, cudaStream_t st) {

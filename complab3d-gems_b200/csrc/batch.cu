@@ -24,14 +24,12 @@ struct clb_batch_s {
     int flow_prec = 0, ade_prec = 0, nm = 1;
     bool has_flow = false, has_ade = false;
     clb::BatchDomain* d_dom = nullptr;
-    int64_t *d_foff = nullptr, *d_aoff = nullptr, *d_joff = nullptr, *d_face_off = nullptr;
     clb::NeumannJob* d_jobs = nullptr;
     clb::BatchTile *d_ftiles = nullptr, *d_atiles = nullptr;
     void* d_sdom = nullptr;       // StreamDomain of every domain
-    clb::NeumannFace* d_faces = nullptr;
+    clb::NeumannTile* d_ntiles = nullptr;
     clb::BatchView view{};
     int64_t flow_nodes = 0, ade_nodes = 0;
-    int neu_grid = 148;
     bool flow_staged = false;  // schedule mode 2 was asked for (the same launches as mode 0)
     // graphs by (flow parity, ade parity, flow, ade, steps per launch (0: per lattice), tile, lag)
     std::map<std::tuple<int, int, int, int, int, int, int>, cudaGraphExec_t> graphs;
@@ -79,15 +77,11 @@ static void batch_free(clb_batch* b) {
     cudaFree(b->d_sync);
     cudaFree(b->d_jbeg);
     cudaFree(b->d_dom);
-    cudaFree(b->d_foff);
-    cudaFree(b->d_aoff);
     cudaFree(b->d_jobs);
-    cudaFree(b->d_joff);
     cudaFree(b->d_ftiles);
     cudaFree(b->d_atiles);
     cudaFree(b->d_sdom);
-    cudaFree(b->d_faces);
-    cudaFree(b->d_face_off);
+    cudaFree(b->d_ntiles);
     if (b->stream) cudaStreamDestroy(b->stream);
 }
 
@@ -126,11 +120,10 @@ clb_status batch_create(clb_handle* const* hs, int n, clb_batch** out) {
     if (!b->has_flow && !b->has_ade) { delete b; return fail(nullptr, CLB_INVALID_ARG, "nothing to step in the batch"); }
     cudaSetDevice(b->device);
     std::vector<BatchDomain> dom((size_t)n);
-    std::vector<int64_t> foff((size_t)n + 1, 0), aoff((size_t)n + 1, 0), joff(1, 0);
+    int64_t flow_nodes = 0, ade_nodes = 0;
     std::vector<NeumannJob> jobs;
     std::vector<BatchTile> ftiles, atiles;
-    std::vector<NeumannFace> faces;
-    std::vector<int64_t> face_off(1, 0);
+    std::vector<NeumannTile> ntiles;
     b->kf.assign((size_t)n, 0);
     b->ka.assign((size_t)n, 0);
     b->jbeg.assign((size_t)n + 1, 0);
@@ -146,7 +139,7 @@ clb_status batch_create(clb_handle* const* hs, int n, clb_batch** out) {
             d.fkw = h->k_west_end;
             d.fke = h->k_east_begin;
             d.fp = h->fp;
-            foff[(size_t)i + 1] = foff[(size_t)i] + h->flow_sp.K;
+            flow_nodes += h->flow_sp.K;
             b->kf[(size_t)i] = h->flow_sp.K;
             for (int64_t k = 0; k < h->flow_sp.K; k += BATCH_FLOW_TILE)
                 ftiles.push_back({i, (int)std::min<int64_t>(BATCH_FLOW_TILE, h->flow_sp.K - k), k});
@@ -165,15 +158,14 @@ clb_status batch_create(clb_handle* const* hs, int n, clb_batch** out) {
             d.mob = (const int*)(h->d_neu + (size_t)h->S * 2 * h->g.plane);  // the mobile-species table
             d.mat = h->d_mat;
             d.n_mobile = h->n_mobile;
-            aoff[(size_t)i + 1] = aoff[(size_t)i] + h->ade_sp.K;
+            ade_nodes += h->ade_sp.K;
             b->ka[(size_t)i] = h->ade_sp.K;
             for (int side = 0; side < 2; ++side) {
                 bool any = false;
                 for (int s = 0; s < h->S; ++s)
                     any = any || (h->ap.slot[s] >= 0 && (side == 0 ? h->ap.ltype[s] : h->ap.rtype[s]) == CLB_NEUMANN);
                 if (!any) continue;
-                faces.push_back({i, side});
-                face_off.push_back(face_off.back() + h->g.plane);
+                for (int p = 0; p < h->g.plane; p += NEUMANN_TILE) ntiles.push_back({i, side, p});
             }
             for (int s = 0; s < h->S; ++s) {
                 const int m = h->ap.slot[s];
@@ -181,7 +173,6 @@ clb_status batch_create(clb_handle* const* hs, int n, clb_batch** out) {
                 for (int side = 0; side < 2; ++side) {
                     if ((side == 0 ? h->ap.ltype[s] : h->ap.rtype[s]) != CLB_NEUMANN) continue;
                     jobs.push_back({i, s, m, side});
-                    joff.push_back(joff.back() + h->g.plane);
                 }
             }
         }
@@ -202,36 +193,27 @@ clb_status batch_create(clb_handle* const* hs, int n, clb_batch** out) {
             alaw[q + 1] = (int)atiles.size();
         }
     }
-    b->flow_nodes = foff.back();
-    b->ade_nodes = aoff.back();
+    b->flow_nodes = flow_nodes;
+    b->ade_nodes = ade_nodes;
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_dom, sizeof(BatchDomain) * n);
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_foff, sizeof(int64_t) * (n + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_aoff, sizeof(int64_t) * (n + 1));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_jobs, sizeof(NeumannJob) * std::max<size_t>(1, jobs.size()));
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_joff, sizeof(int64_t) * joff.size());
     if (e == cudaSuccess) e = cudaMalloc(&b->d_jbeg, sizeof(int) * (n + 1));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_ftiles, sizeof(BatchTile) * std::max<size_t>(1, ftiles.size()));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_atiles, sizeof(BatchTile) * std::max<size_t>(1, atiles.size()));
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_faces, sizeof(NeumannFace) * std::max<size_t>(1, faces.size()));
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_face_off, sizeof(int64_t) * face_off.size());
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_ntiles, sizeof(NeumannTile) * std::max<size_t>(1, ntiles.size()));
     if (e == cudaSuccess && !ftiles.empty())
         e = cudaMemcpy(b->d_ftiles, ftiles.data(), sizeof(BatchTile) * ftiles.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && !atiles.empty())
         e = cudaMemcpy(b->d_atiles, atiles.data(), sizeof(BatchTile) * atiles.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && !faces.empty())
-        e = cudaMemcpy(b->d_faces, faces.data(), sizeof(NeumannFace) * faces.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = cudaMemcpy(b->d_face_off, face_off.data(), sizeof(int64_t) * face_off.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && !ntiles.empty())
+        e = cudaMemcpy(b->d_ntiles, ntiles.data(), sizeof(NeumannTile) * ntiles.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_sync, sizeof(int) * (2 + (size_t)PERSIST_MAX_STEPS * 3 * n));
     if (e == cudaSuccess) e = cudaMemset(b->d_sync, 0, sizeof(int) * (2 + (size_t)PERSIST_MAX_STEPS * 3 * n));
     if (e == cudaSuccess) e = cudaMemcpy(b->d_jbeg, b->jbeg.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(b->d_dom, dom.data(), sizeof(BatchDomain) * n, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(b->d_foff, foff.data(), sizeof(int64_t) * (n + 1), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(b->d_aoff, aoff.data(), sizeof(int64_t) * (n + 1), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && !jobs.empty())
         e = cudaMemcpy(b->d_jobs, jobs.data(), sizeof(NeumannJob) * jobs.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(b->d_joff, joff.data(), sizeof(int64_t) * joff.size(), cudaMemcpyHostToDevice);
     // the batch's own stream does not wait for the legacy stream's uploads
     if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
     if (e != cudaSuccess) {
@@ -240,11 +222,8 @@ clb_status batch_create(clb_handle* const* hs, int n, clb_batch** out) {
         return fail(nullptr, CLB_CUDA_ERROR, std::string("batch set-up: ") + cudaGetErrorString(e));
     }
     b->view.dom = b->d_dom;
-    b->view.foff = b->d_foff;
-    b->view.aoff = b->d_aoff;
     b->view.ndom = n;
     b->view.jobs = b->d_jobs;
-    b->view.joff = b->d_joff;
     b->view.njobs = (int)jobs.size();
     b->view.ftiles = b->d_ftiles;
     b->view.nft = (int)ftiles.size();
@@ -252,10 +231,8 @@ clb_status batch_create(clb_handle* const* hs, int n, clb_batch** out) {
     for (int q = 0; q < 5; ++q) b->view.alaw[q] = alaw[q];
     b->view.sdom = b->d_sdom;
     b->view.max_mobile = max_mobile;
-    b->view.faces = b->d_faces;
-    b->view.foff_faces = b->d_face_off;
-    b->view.nfaces = (int)faces.size();
-    b->neu_grid = std::max<int64_t>(1, std::min<int64_t>((face_off.back() + 255) / 256, b->num_sms * 4));
+    b->view.ntiles = b->d_ntiles;
+    b->view.nnt = (int)ntiles.size();
     b->resident = batch_persistent_resident(b->has_ade ? b->ade_prec : b->flow_prec, b->nm, b->minb);
     if (b->has_flow && b->has_ade && b->flow_prec != b->ade_prec) b->persistent = false;  // one storage type per launch
     *out = b;
@@ -340,7 +317,7 @@ static clb_status persist_launch(clb_batch* b, int steps, int fodd, int aodd, bo
 static void batch_launch_step(clb_batch* b, int fodd, int aodd, bool flow, bool ade) {
     if (flow) launch_flow_batch(b->view, b->flow_prec, fodd != 0, bstream(b));
     if (ade) {
-        launch_neumann_batch(b->view, b->ade_prec, aodd != 0, b->neu_grid, bstream(b));
+        launch_neumann_batch(b->view, b->ade_prec, aodd != 0, bstream(b));
         launch_ade_batch(b->view, b->ade_prec, aodd != 0, bstream(b));
     }
 }

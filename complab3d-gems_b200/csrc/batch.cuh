@@ -46,18 +46,16 @@ struct BatchTile {
 // flow 96 domains 134.8 at 256 nodes, 135.4 at 512.
 constexpr int BATCH_FLOW_TILE = 256;
 constexpr int BATCH_ADE_TILE = 128;
-// One x-face of one domain that at least one mobile species treats as Neumann
-struct NeumannFace {
-    int d, side;
+// 128 pixels of an x-face of one domain that at least one mobile species treats as Neumann
+struct NeumannTile {
+    int d, side, first;
 };
+constexpr int NEUMANN_TILE = 128;
 
 struct BatchView {
     const BatchDomain* dom;
-    const int64_t* foff;  // [ndom + 1] prefix sums of the flow node counts
-    const int64_t* aoff;  // [ndom + 1] prefix sums of the species node counts
     int ndom;
     const NeumannJob* jobs;
-    const int64_t* joff;  // [njobs + 1] prefix sums of the plane sizes
     int njobs;
     const BatchTile* ftiles;  // flow tiles, domain by domain
     int nft;
@@ -65,9 +63,8 @@ struct BatchView {
     int alaw[5];              // the tiles of form q are atiles[alaw[q] .. alaw[q + 1])
     const void* sdom;         // StreamDomain of every domain
     int max_mobile;
-    const NeumannFace* faces;
-    const int64_t* foff_faces;  // [nfaces + 1] prefix sums of the face sizes
-    int nfaces;
+    const NeumannTile* ntiles;
+    int nnt;
 };
 
 constexpr int BATCH_MAX_DOMAINS = 2048;
@@ -104,8 +101,8 @@ void launch_flow_batch(const BatchView& B, int prec, bool odd, cudaStream_t st);
 // streamed form of each handle's law)
 void launch_ade_batch(const BatchView& B, int prec, bool odd, cudaStream_t st);
 cudaError_t stream_domains(clb_handle* const* hs, int n, int prec, void** dev, std::vector<int>& form);
+void launch_neumann_batch(const BatchView& B, int prec, bool odd, cudaStream_t st);
 // ade.cu
-void launch_neumann_batch(const BatchView& B, int prec, bool odd, int grid, cudaStream_t st);
 // the persistent schedule: one launch runs the whole item table (nm: species register bucket 1, 2, 4,
 // 8 or 16)
 void launch_batch_persistent(const PersistView& V, int prec, int nm, int minb, int blocks_per_sm, int num_sms,

@@ -405,6 +405,8 @@ void ade_refresh_neumann(clb_handle* h);
 // (no abiotic law, dissolution, gate or rate-law file)
 bool ade_streams(const AdeParams& P);
 void launch_ade_stream(clb_handle* h, bool odd);
+// the stored densities of every Neumann plane before a step of the given parity
+void launch_ade_neumann(clb_handle* h, bool odd);
 // all of `steps` steps in cooperative launches, where the lattice is small enough; false: not taken
 bool launch_ade_multi(clb_handle* h, int steps, cudaError_t& e);
 void ade_free(clb_handle* h);
