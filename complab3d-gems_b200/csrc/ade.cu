@@ -1260,7 +1260,7 @@ static int ade_grid_for(const void* kern, int smem, int num_sms, int threads, in
 }
 
 template <typename TS, typename TC, bool ODD>
-static void launch_ade_t(clb_handle* h) {
+static void launch_ade_t(clb_handle* h, bool after) {
     const int nm = h->n_mobile;
     const int nb = h->S;  // register bucket covers every species (mobile first, then immobile)
     TS* g = (TS*)h->d_g;
@@ -1288,7 +1288,7 @@ static void launch_ade_t(clb_handle* h) {
     auto go = [&](auto NM, auto EXT) {
         constexpr int B = decltype(NM)::value, E = decltype(EXT)::value;
         if (pipe(NM, EXT)) return;
-        if constexpr (E == 0) launch_ade_stream(h, ODD);
+        if constexpr (E == 0) launch_ade_stream(h, ODD, after);
         else staged(k_ade_aa<TS, TC, ODD, B, E>, ade_slot_bytes<TC, B>(), ODD ? ADE_RESIDENT : ADE_RESIDENT_EVEN);
     };
     // EXT: 0 the compiled biotic laws alone; 1 with the abiotic block, dissolution and the
@@ -1311,10 +1311,11 @@ static void launch_ade_t(clb_handle* h) {
 // The stored densities are those after the latest stream; they are recomputed lazily, once per
 // transport iteration, so that a readback or a change of the material map between two steps
 // (clb_geometry_update refreshes them before it converts voxels) does not alter them.
-static void refresh_neumann(clb_handle* h) {
-    if (h->neu_iter == h->ade_iters) return;
+// True where it launched the planes' kernel.
+static bool refresh_neumann(clb_handle* h, bool after = false) {
+    if (h->neu_iter == h->ade_iters) return false;
     h->neu_iter = h->ade_iters;
-    launch_ade_neumann(h, (h->ade_iters & 1) != 0);
+    return launch_ade_neumann(h, (h->ade_iters & 1) != 0, after);
 }
 
 // ------------------------------------------------------------------ persistent batched steps
@@ -1558,20 +1559,24 @@ clb_status ade_step(clb_handle* h, int n) {
             return cuda_check(h, e, "ade steps");
         }
     }
+    const bool streamed = ade_streams(h->ap) && !h->ade_pipe;
+    bool after = false;  // the stream's latest work is a streamed step or its planes, launched by this call
     for (int k = 0; k < n; ++k) {
         const bool odd = (h->ade_iters & 1) != 0;
         if (h->ap.dis_on) {
             clb_status st = dissolution_pre_step(h);
             if (st != CLB_OK) return st;
         }
-        refresh_neumann(h);
+        if (refresh_neumann(h, after)) after = streamed;
         switch (h->ade_prec) {
-            case CLB_F64: if (odd) launch_ade_t<double, double, true>(h); else launch_ade_t<double, double, false>(h); break;
-            case CLB_F32: if (odd) launch_ade_t<float, float, true>(h); else launch_ade_t<float, float, false>(h); break;
-            default: if (odd) launch_ade_t<__half, float, true>(h); else launch_ade_t<__half, float, false>(h); break;
+            case CLB_F64: if (odd) launch_ade_t<double, double, true>(h, after); else launch_ade_t<double, double, false>(h, after); break;
+            case CLB_F32: if (odd) launch_ade_t<float, float, true>(h, after); else launch_ade_t<float, float, false>(h, after); break;
+            default: if (odd) launch_ade_t<__half, float, true>(h, after); else launch_ade_t<__half, float, false>(h, after); break;
         }
         h->ade_iters += 1;
+        after = streamed;
         if (h->spec_mode != CLB_SPEC_OFF) {
+            after = false;
             clb_status st = speciation_step(h);
             if (st != CLB_OK) return st;
         }

@@ -34,7 +34,7 @@ constexpr int stream_blocks() { return sizeof(TC) == 4 && U == 1 ? 10 : 8; }
 template <typename TS, typename TC, bool ODD, int U, int LAW>
 __global__ void __launch_bounds__(STREAM_THREADS, (stream_blocks<TC, U>()))
     k_ade_stream(TS* __restrict__ g, double* __restrict__ imm, double* __restrict__ bio, const TC* __restrict__ u,
-                 const SparseView S, const double* __restrict__ neu, const AdeStep<TC> P, int64_t kw, int64_t ke) {
+                 const SparseView S, const double* neu, const AdeStep<TC> P, int64_t kw, int64_t ke) {
     extern __shared__ __align__(16) unsigned char stream_smem[];
     const int64_t k = (int64_t)blockIdx.x * STREAM_THREADS + threadIdx.x;
     ade_stream_node<TS, TC, ODD, U, LAW, STREAM_THREADS>(g, imm, bio, u, S, neu, P, kw, ke, stream_smem, k, k < S.K);
@@ -45,15 +45,15 @@ bool ade_streams(const AdeParams& P) {
 }
 
 template <typename TS, typename TC, bool ODD>
-static void launch_stream_t(clb_handle* h) {
+static void launch_stream_t(clb_handle* h, bool after) {
     const SparseView S = view_of(h->ade_sp);
     const AdeStep<TC> P = ade_step_params<TC>(h->ap, h->n_mobile);
     const unsigned grid = (unsigned)std::max<int64_t>(1, (S.K + STREAM_THREADS - 1) / STREAM_THREADS);
     const StreamLaw law = stream_law(P, sizeof(TS));
     const size_t sm = (size_t)stream_bytes<TC>(law, h->n_mobile) * STREAM_THREADS;
     auto go = [&](auto kern) {
-        kern<<<grid, STREAM_THREADS, sm, h->stream>>>((TS*)h->d_g, h->d_imm, h->d_bio, (const TC*)h->d_u, S, h->d_neu, P,
-                                                      h->ade_west_end, h->ade_east_begin);
+        launch_step(after, kern, grid, STREAM_THREADS, sm, h->stream, (TS*)h->d_g, h->d_imm, h->d_bio, (const TC*)h->d_u, S,
+                    h->d_neu, P, h->ade_west_end, h->ade_east_begin);
     };
     constexpr int U = stream_width<TC>();
     const bool one = h->n_mobile == 1;
@@ -70,12 +70,12 @@ static void launch_stream_t(clb_handle* h) {
     }
 }
 
-void launch_ade_stream(clb_handle* h, bool odd) {
+void launch_ade_stream(clb_handle* h, bool odd, bool after) {
     ++h->launches;
     switch (h->ade_prec) {
-        case CLB_F64: if (odd) launch_stream_t<double, double, true>(h); else launch_stream_t<double, double, false>(h); break;
-        case CLB_F32: if (odd) launch_stream_t<float, float, true>(h); else launch_stream_t<float, float, false>(h); break;
-        default: if (odd) launch_stream_t<__half, float, true>(h); else launch_stream_t<__half, float, false>(h); break;
+        case CLB_F64: if (odd) launch_stream_t<double, double, true>(h, after); else launch_stream_t<double, double, false>(h, after); break;
+        case CLB_F32: if (odd) launch_stream_t<float, float, true>(h, after); else launch_stream_t<float, float, false>(h, after); break;
+        default: if (odd) launch_stream_t<__half, float, true>(h, after); else launch_stream_t<__half, float, false>(h, after); break;
     }
 }
 
@@ -89,16 +89,19 @@ void launch_ade_stream(clb_handle* h, bool odd) {
 // the dense neighbour lookups (five dependent reads, 64-bit divisions, a search for the batch's
 // domain) 12.7 and 13.4.
 template <typename TS, typename TC, bool ODD>
-__device__ __forceinline__ void neumann_pixel(const TS* __restrict__ g, const SparseView& S, const int8_t* dyn, int nx, int plane,
-                                              int side, int p, int s, double* __restrict__ neu) {
+__device__ __forceinline__ void neumann_pixel(const TS* g, const SparseView& S, const int8_t* dyn, int nx, int plane,
+                                              int side, int p, int s, bool on, double* neu) {
     const int64_t nb = side == 0 ? p : (int64_t)(nx - 1) * plane + p, ni = side == 0 ? nb + plane : nb - plane;
-    const int kb = S.idx_of[nb], ki = S.idx_of[ni];
-    if (kb < 0 || ki < 0) return;
-    const int cb = S.code[kb], ci = S.code[ki];
+    const int kb = on ? S.idx_of[nb] : -1, ki = on ? S.idx_of[ni] : -1;
     uint32_t off[7];
-    stream_slots<ODD>(S, ki, S.meta[ki], off);
-    const int db = dyn[cb], di = dyn[ci];
-    if (!(db == ADE_PORE || db == ADE_BIO) || !(di == ADE_PORE || di == ADE_BIO)) return;
+    on = kb >= 0 && ki >= 0;
+    if (on) {
+        const int db = dyn[S.code[kb]], di = dyn[S.code[ki]];
+        stream_slots<ODD>(S, ki, S.meta[ki], off);
+        on = (db == ADE_PORE || db == ADE_BIO) && (di == ADE_PORE || di == ADE_BIO);
+    }
+    step_wait();
+    if (!on) return;
     const TS* f = g + (int64_t)s * S.SS;
     TC pop[7];
 #pragma unroll
@@ -118,14 +121,13 @@ struct NeumannPlanes {
 };
 
 template <typename TS, typename TC, bool ODD>
-__global__ void __launch_bounds__(STREAM_THREADS) k_neumann(const TS* __restrict__ g, const SparseView S, const NeumannPlanes J,
-                                                            double* __restrict__ neu) {
+__global__ void __launch_bounds__(STREAM_THREADS) k_neumann(const TS* g, const SparseView S, const NeumannPlanes J, double* neu) {
     const int p = blockIdx.x * STREAM_THREADS + threadIdx.x, side = blockIdx.y, j = blockIdx.z;
-    if (p >= J.plane || j >= J.n[side]) return;
-    neumann_pixel<TS, TC, ODD>(g, S, J.dyn, J.nx, J.plane, side, p, J.s[side][j], neu);
+    const bool on = p < J.plane && j < J.n[side];
+    neumann_pixel<TS, TC, ODD>(g, S, J.dyn, J.nx, J.plane, side, p, on ? J.s[side][j] : 0, on, neu);
 }
 
-void launch_ade_neumann(clb_handle* h, bool odd) {
+bool launch_ade_neumann(clb_handle* h, bool odd, bool after) {
     NeumannPlanes J;
     J.nx = h->g.nx;
     J.plane = h->g.plane;
@@ -135,19 +137,20 @@ void launch_ade_neumann(clb_handle* h, bool odd) {
         if (h->ap.rtype[s] == CLB_NEUMANN) J.s[1][J.n[1]++] = (int8_t)s;
     }
     const int most = std::max(J.n[0], J.n[1]);
-    if (most == 0) return;
+    if (most == 0) return false;
     std::memcpy(J.dyn, h->ap.dyn, sizeof(J.dyn));
     const dim3 grid((unsigned)((h->g.plane + STREAM_THREADS - 1) / STREAM_THREADS), 2, (unsigned)most);
     ++h->launches;
 #define CLB_NEU(TS, TC)                                                                                                    \
-    if (odd) k_neumann<TS, TC, true><<<grid, STREAM_THREADS, 0, h->stream>>>((const TS*)h->d_g, view_of(h->ade_sp), J, h->d_neu); \
-    else k_neumann<TS, TC, false><<<grid, STREAM_THREADS, 0, h->stream>>>((const TS*)h->d_g, view_of(h->ade_sp), J, h->d_neu);
+    launch_step(after, odd ? k_neumann<TS, TC, true> : k_neumann<TS, TC, false>, grid, STREAM_THREADS, 0, h->stream,                 \
+                (const TS*)h->d_g, view_of(h->ade_sp), J, h->d_neu);
     switch (h->ade_prec) {
         case CLB_F64: CLB_NEU(double, double); break;
         case CLB_F32: CLB_NEU(float, float); break;
         default: CLB_NEU(__half, float); break;
     }
 #undef CLB_NEU
+    return true;
 }
 
 // ------------------------------------------------------------------ many steps of a small lattice
@@ -368,8 +371,8 @@ __global__ void __launch_bounds__(STREAM_THREADS) k_neumann_batch(const NeumannT
     const NeumannTile T = tiles[blockIdx.x];
     const StreamDomain<TC>& D = dom[T.d];
     const int s = blockIdx.y, p = T.first + (int)threadIdx.x;
-    if (p >= D.P.plane || s >= D.P.n_mobile || (T.side == 0 ? D.P.ltype[s] : D.P.rtype[s]) != CLB_NEUMANN) return;
-    neumann_pixel<TS, TC, ODD>((const TS*)D.g, D.S, D.P.dyn, (int)(D.P.N / D.P.plane), D.P.plane, T.side, p, s,
+    const bool on = p < D.P.plane && s < D.P.n_mobile && (T.side == 0 ? D.P.ltype[s] : D.P.rtype[s]) == CLB_NEUMANN;
+    neumann_pixel<TS, TC, ODD>((const TS*)D.g, D.S, D.P.dyn, (int)(D.P.N / D.P.plane), D.P.plane, T.side, p, s, on,
                                const_cast<double*>(D.neu));
 }
 

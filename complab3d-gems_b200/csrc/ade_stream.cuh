@@ -14,6 +14,7 @@
 
 #include "flow_node.cuh"
 #include "kinetics.cuh"
+#include "step_chain.cuh"
 #include "tma.cuh"
 
 #include <cstring>
@@ -393,8 +394,8 @@ __device__ __forceinline__ void ade_stream_species(TS* g, double* imm, double* b
 template <typename TS, typename TC, bool ODD, int U, int LAW, int T>
 __device__ __forceinline__ void ade_stream_node(TS* __restrict__ g, double* __restrict__ imm, double* __restrict__ bio,
                                                 const TC* __restrict__ u, const SparseView& S,
-                                                const double* __restrict__ neu, const AdeStep<TC>& P, int64_t kw,
-                                                int64_t ke, unsigned char* smem, int64_t k, bool on) {
+                                                const double* neu, const AdeStep<TC>& P, int64_t kw, int64_t ke,
+                                                unsigned char* smem, int64_t k, bool on) {
     StreamNode<TC> A = {};
     uint32_t off[7] = {0, 0, 0, 0, 0, 0, 0};
     if (on) {
@@ -402,6 +403,7 @@ __device__ __forceinline__ void ade_stream_node(TS* __restrict__ g, double* __re
         A = stream_node<TC, LAW>(S, P, u, k);
         stream_slots<ODD>(S, k, mt, off);
     }
+    step_wait();
     ade_stream_species<TS, TC, U, LAW, T, true>(g, imm, bio, S, P, kw, ke, smem, k, A, off, on, [&](int s, bool west) {
         return neu[((int64_t)s * 2 + (west ? 0 : 1)) * P.plane + S.node[k] % P.plane];
     });

@@ -404,9 +404,10 @@ void ade_refresh_neumann(clb_handle* h);
 // ade_stream.cu: the step with every species streamed through registers, for the laws that allow it
 // (no abiotic law, dissolution, gate or rate-law file)
 bool ade_streams(const AdeParams& P);
-void launch_ade_stream(clb_handle* h, bool odd);
-// the stored densities of every Neumann plane before a step of the given parity
-void launch_ade_neumann(clb_handle* h, bool odd);
+// after: as launch_step (step_chain.cuh)
+void launch_ade_stream(clb_handle* h, bool odd, bool after);
+// the stored densities of every Neumann plane before a step of the given parity; false: there is none
+bool launch_ade_neumann(clb_handle* h, bool odd, bool after);
 // all of `steps` steps in cooperative launches, where the lattice is small enough; false: not taken
 bool launch_ade_multi(clb_handle* h, int steps, cudaError_t& e);
 void ade_free(clb_handle* h);

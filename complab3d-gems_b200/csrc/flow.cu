@@ -29,6 +29,7 @@
 #include "batch.cuh"
 #include "flow_node.cuh"
 #include "grid_sync.cuh"
+#include "step_chain.cuh"
 #include "tma.cuh"
 
 #include <algorithm>
@@ -405,6 +406,7 @@ __device__ __forceinline__ double flow_stream_node(TS* __restrict__ f, const Spa
         }
     }
     const int dyn = P.dyn[M.code];
+    step_wait();
     if (dyn == DYN_BB) return 0.0;  // a stored bounce-back node: the identity on AA slots
     double e = 0;
     TC g[19];
@@ -430,6 +432,7 @@ __global__ void __launch_bounds__(STREAM_FLOW_THREADS, (stream_flow_blocks<TS>()
     // round trip of its own
     const int settled = ENERGY && trace ? tr->converged : 0;
     const int64_t k = (int64_t)blockIdx.x * STREAM_FLOW_THREADS + threadIdx.x;
+    if (k >= S.K) step_wait();
     double e = k < S.K ? flow_stream_node<TS, TC, ODD>(f, S, P, k, k_west_end, k_east_begin, settled) : 0.0;
     if (ENERGY) {
 #pragma unroll
@@ -993,7 +996,7 @@ static bool flow_streams(const clb_handle* h, bool trace) {
 
 // One step. The streamed step forms the stored energy, and counts `count` iterations, only where count is
 // not 0; the kernels a tuning key selects do both at every step.
-static void launch_flow(clb_handle* h, bool odd, int trace, int count) {
+static void launch_flow(clb_handle* h, bool odd, int trace, int count, bool after) {
     ++h->launches;  // one step launch per call
     const FlowParams& P = h->fp;
     const SparseView S = view_of(h->flow_sp);
@@ -1002,9 +1005,8 @@ static void launch_flow(clb_handle* h, bool odd, int trace, int count) {
         const unsigned g = (unsigned)std::max<int64_t>(1, flow_tiles(h));
         auto go = [&](auto kern, auto* ts) {
             using TS = std::remove_pointer_t<decltype(ts)>;
-            kern<<<g, STREAM_FLOW_THREADS, 0, h->stream>>>((TS*)h->d_f, S, P, h->d_tracer,
-                                                           h->d_partials + h->partial_cap, trace, h->k_west_end,
-                                                           h->k_east_begin);
+            launch_step(after, kern, g, STREAM_FLOW_THREADS, 0, h->stream, (TS*)h->d_f, S, P, h->d_tracer,
+                        h->d_partials + h->partial_cap, trace, h->k_west_end, h->k_east_begin);
         };
 #define CLB_STREAM(TS, TC)                                                                                \
     if (odd) count ? go(k_flow_stream<TS, TC, true, true>, (TS*)nullptr) : go(k_flow_stream<TS, TC, true, false>, (TS*)nullptr); \
@@ -1105,7 +1107,7 @@ clb_status flow_step(clb_handle* h, int n, bool trace, double eps) {
         return CLB_OK;
     }
     for (int k = 0; k < n; ++k) {
-        launch_flow(h, (h->flow_iters & 1) != 0, trace ? 1 : 0, trace ? 1 : (k + 1 == n ? n : 0));
+        launch_flow(h, (h->flow_iters & 1) != 0, trace ? 1 : 0, trace ? 1 : (k + 1 == n ? n : 0), k > 0 && !trace && flow_streams(h, false));
         h->flow_iters += 1;
     }
     return cuda_check(h, cudaGetLastError(), "flow step");
