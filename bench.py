@@ -93,8 +93,6 @@ def step_kernels(tuned, precision):
     """Names of the two AA-step kernels the flow step ran (the autotuner's choice, else the library's
     default)."""
     choice = tuned.split("->")[-1] if "->" in tuned else "stream"
-    if "multi" in choice:
-        return "k_flow_multi (many AA steps per launch, mean per step)"
     if "stream" in choice:
         return "k_flow_stream (AA even/odd steps, mean per launch)"
     even = "k_flow_even_tma" if "tma=1" in choice else "k_flow_aa<even>"
@@ -331,7 +329,7 @@ def bench_d3q7(clb, workloads, torch, local, peak, steps=60, warmup=5, scale=1.0
             "steps": steps,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "algorithmic_bytes_per_node": alg_node, "biomass_flagged_fraction": flagged,
-                         "kernel": "k_ade_aa (all species fused)"}}
+                         "kernel": "k_ade_stream (all species fused)"}}
 
 
 def bench_precision(clb, workloads, torch, local, steps=300, warmup=20):
@@ -749,7 +747,7 @@ def main():
             "traffic": traffic_per_launch("k_ade_aa_f32_pack256cube_8species"), "peak_source": peak_kind,
             "algorithmic_bytes_per_launch": alg_node * n_open, "algorithmic_bytes_per_node": alg_node,
             "biomass_flagged_fraction": [bio_start[1], bio_end[1]],
-            "kernel": "k_ade_aa (all 8 species fused, even/odd AA steps) + k_ade_neumann, the fused transport "
+            "kernel": "k_ade_stream (all 8 species fused, even/odd AA steps) + k_neumann, the fused transport "
                       "step; mean device time per iteration from CUDA events on the handle's stream",
             "share_of_step": ms_transport / sum(ms_blocks)}
 

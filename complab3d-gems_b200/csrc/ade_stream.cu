@@ -156,8 +156,8 @@ bool launch_ade_neumann(clb_handle* h, bool odd, bool after) {
 // ------------------------------------------------------------------ many steps of a small lattice
 
 // `steps` steps in one cooperative launch, for lattices small enough that a step is mostly latency (two
-// launches, the Neumann planes' and the step's, their ramp-up and the metadata): the resident threads
-// keep (ONE) or walk their nodes, and the blocks meet at a grid-wide barrier between steps.
+// launches, the Neumann planes' and the step's, their ramp-up and the metadata): every node has a resident
+// thread that keeps its slots of both parities, and the blocks meet at a grid-wide barrier between steps.
 //
 // A Neumann face imposes the density its node's inner neighbour has before the step, which the
 // neighbour's own update overwrites. So the thread of such a face node takes the inner neighbour too: the
@@ -165,7 +165,7 @@ bool launch_ade_neumann(clb_handle* h, bool odd, bool after) {
 // leaves it out. (nx >= 4, so that no inner node belongs to two faces.)
 constexpr int STREAM_MULTI_THREADS = 256;
 
-template <typename TS, typename TC, int U, int LAW, bool ONE>
+template <typename TS, typename TC, int U, int LAW>
 __global__ void __launch_bounds__(STREAM_MULTI_THREADS, 2)
     k_ade_stream_multi(TS* g, double* imm, double* bio, const TC* u, const SparseView S, const double* neu, const AdeStep<TC> P,
                        int64_t kw, int64_t ke, int neumann, int steps, int odd, GridSync* gs, int* err) {
@@ -214,12 +214,12 @@ __global__ void __launch_bounds__(STREAM_MULTI_THREADS, 2)
         if (odd_step) run(N.odd, I.odd);
         else run(N.even, I.even);
     };
-    const int64_t k0 = (int64_t)blockIdx.x * T + threadIdx.x, stride = (int64_t)gridDim.x * T;
+    const int64_t k = (int64_t)blockIdx.x * T + threadIdx.x;
     Node N = {}, I = {};
     int64_t kp = -1;
     bool mine = false;
-    // a node next to a face whose partner exists belongs to the partner's thread
-    auto place = [&](int64_t k) {
+    if (k < S.K) {
+        // a node next to a face whose partner exists belongs to the partner's thread
         const bool face = k < kw || k >= ke;
         kp = partner(k);
         mine = face || kp < 0;
@@ -228,18 +228,10 @@ __global__ void __launch_bounds__(STREAM_MULTI_THREADS, 2)
             N = load(k);
             if (kp >= 0) I = load(kp);
         }
-    };
-    if (ONE && k0 < S.K) place(k0);
+    }
     for (int t = 0; t < steps; ++t) {
         const bool odd_step = ((odd + t) & 1) != 0;
-        if (ONE) {
-            if (mine) step(k0, N, kp, I, odd_step);
-        } else {
-            for (int64_t k = k0; k < S.K; k += stride) {
-                place(k);
-                if (mine) step(k, N, kp, I, odd_step);
-            }
-        }
+        if (mine) step(k, N, kp, I, odd_step);
         if (!grid_barrier(gs, (unsigned)t + 1)) {
             if (threadIdx.x == 0) atomicExch(err, 1);
             return;
@@ -247,19 +239,21 @@ __global__ void __launch_bounds__(STREAM_MULTI_THREADS, 2)
     }
 }
 
-// Lattices whose steps go many to a launch, by nodes and by nodes x mobile species. us per step, a
-// launch per step -> many steps per launch (FP64; FP32):
-//   one species:     27 k nodes 10.4 -> 3.0; 10.3 -> 2.8    91 k 12.3 -> 6.6; 11.3 -> 6.2    214 k 14.4 -> 9.0; 12.3 -> 8.2
-//                   482 k 18.5 -> 15.4; 14.8 -> 14.0
-//   three (Monod):   27 k 14.4 -> 6.2; 12.9 -> 5.6          214 k 22.6 -> 16.8; 18.0 -> 13.9  482 k 42 -> 45; 24.9 -> 25.1
-//   eight (dual):    27 k 24.7 -> 15.5; 21.0 -> 13.1         91 k 30.8 -> 28.6; 23.8 -> 22.3  214 k 56.3 -> 56.8; 33.8 -> 31.5
-constexpr int64_t STREAM_MULTI_NODES = 400000, STREAM_MULTI_VALUES = 1500000;
+// Lattices whose steps go many to a launch: up to two mobile species and by nodes x species, since a
+// chained launch per step has the whole chip per species group where this one has a barrier. us per step, chained
+// launches -> many steps per launch (FP64; FP32):
+//   one species:   11 k nodes 7.4 -> 3.2; 4.9 -> 3.0    53 k 7.6 -> 3.7; 4.8 -> 3.4    76 k 7.4 -> 5.7; 4.9 -> 5.5
+//   two (Monod):   11 k 7.5 -> 4.4; 4.8 -> 4.2          27 k 7.3 -> 4.6; 4.9 -> 4.2    43 k 7.4 -> 5.7; 4.9 -> 5.0
+//   three (Monod): 11 k 5.8 -> 5.3; 5.3 -> 5.2          27 k 7.5 -> 6.2; 5.5 -> 5.6    43 k 6.3 -> 7.8; 5.6 -> 6.7
+//   four (dual):   11 k 7.3 -> 8.7; 6.7 -> 7.7          27 k 7.9 -> 8.9; 6.7 -> 8.0
+constexpr int STREAM_MULTI_SPECIES = 2;
+constexpr int64_t STREAM_MULTI_VALUES = 60000;
 constexpr int STREAM_MULTI_STEPS = 1024, STREAM_MULTI_MIN_STEPS = 3;
 
 template <typename TS, typename TC>
 static bool launch_stream_multi_t(clb_handle* h, int steps, cudaError_t& e) {
     SparseView S = view_of(h->ade_sp);
-    if (S.K < 1 || S.K > STREAM_MULTI_NODES || S.K * std::max(1, h->n_mobile) > STREAM_MULTI_VALUES) return false;
+    if (S.K < 1 || h->n_mobile > STREAM_MULTI_SPECIES || S.K * std::max(1, h->n_mobile) > STREAM_MULTI_VALUES) return false;
     AdeStep<TC> P = ade_step_params<TC>(h->ap, h->n_mobile);
     const StreamLaw law = stream_law(P, sizeof(TS));
     const size_t sm = (size_t)stream_bytes<TC>(law, h->n_mobile) * STREAM_MULTI_THREADS;
@@ -269,15 +263,12 @@ static bool launch_stream_multi_t(clb_handle* h, int steps, cudaError_t& e) {
         if (P.ltype[s] == CLB_NEUMANN) neumann |= 1;
         if (P.rtype[s] == CLB_NEUMANN) neumann |= 2;
     }
-    auto go = [&](auto one, auto walk) {
+    auto go = [&](auto kern) {
         const int64_t need = (S.K + STREAM_MULTI_THREADS - 1) / STREAM_MULTI_THREADS;
-        int per1 = 0, perw = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per1, one, STREAM_MULTI_THREADS, sm) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perw, walk, STREAM_MULTI_THREADS, sm) != cudaSuccess)
+        int per = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, STREAM_MULTI_THREADS, sm) != cudaSuccess ||
+            need > (int64_t)per * h->num_sms)
             return false;
-        const bool fits = need <= (int64_t)per1 * h->num_sms;
-        const unsigned grid = (unsigned)(fits ? need : (int64_t)perw * h->num_sms);
-        if (grid == 0) return false;
         TS* g = (TS*)h->d_g;
         const TC* u = (const TC*)h->d_u;
         const double* neu = h->d_neu;
@@ -290,8 +281,7 @@ static bool launch_stream_multi_t(clb_handle* h, int steps, cudaError_t& e) {
                             &gs, &err};
             if ((e = cudaMemsetAsync(gs, 0, sizeof(GridSync), h->stream)) != cudaSuccess) return true;
             ++h->launches;
-            e = cudaLaunchCooperativeKernel(fits ? (const void*)one : (const void*)walk, dim3(grid), dim3(STREAM_MULTI_THREADS), args,
-                                            sm, h->stream);
+            e = cudaLaunchCooperativeKernel((const void*)kern, dim3((unsigned)need), dim3(STREAM_MULTI_THREADS), args, sm, h->stream);
             if (e != cudaSuccess) return true;
         }
         return true;
@@ -299,15 +289,15 @@ static bool launch_stream_multi_t(clb_handle* h, int steps, cudaError_t& e) {
     constexpr int U = stream_width<TC>();
     const bool single = h->n_mobile == 1;
     if (law == STREAM_NONE)
-        return single ? go(k_ade_stream_multi<TS, TC, 1, STREAM_NONE, true>, k_ade_stream_multi<TS, TC, 1, STREAM_NONE, false>)
-                      : go(k_ade_stream_multi<TS, TC, U, STREAM_NONE, true>, k_ade_stream_multi<TS, TC, U, STREAM_NONE, false>);
+        return single ? go(k_ade_stream_multi<TS, TC, 1, STREAM_NONE>)
+                      : go(k_ade_stream_multi<TS, TC, U, STREAM_NONE>);
     if (law == STREAM_SEPARABLE)
-        return single ? go(k_ade_stream_multi<TS, TC, 1, STREAM_SEPARABLE, true>, k_ade_stream_multi<TS, TC, 1, STREAM_SEPARABLE, false>)
-                      : go(k_ade_stream_multi<TS, TC, U, STREAM_SEPARABLE, true>, k_ade_stream_multi<TS, TC, U, STREAM_SEPARABLE, false>);
+        return single ? go(k_ade_stream_multi<TS, TC, 1, STREAM_SEPARABLE>)
+                      : go(k_ade_stream_multi<TS, TC, U, STREAM_SEPARABLE>);
     if (law == STREAM_DUAL_AHEAD)
-        return go(k_ade_stream_multi<TS, TC, U, STREAM_DUAL_AHEAD, true>, k_ade_stream_multi<TS, TC, U, STREAM_DUAL_AHEAD, false>);
+        return go(k_ade_stream_multi<TS, TC, U, STREAM_DUAL_AHEAD>);
     if constexpr (sizeof(TS) >= 4)
-        return go(k_ade_stream_multi<TS, TC, U, STREAM_DUAL_AFTER, true>, k_ade_stream_multi<TS, TC, U, STREAM_DUAL_AFTER, false>);
+        return go(k_ade_stream_multi<TS, TC, U, STREAM_DUAL_AFTER>);
     return false;
 }
 

@@ -453,14 +453,14 @@ __global__ void __launch_bounds__(STREAM_FLOW_THREADS, (stream_flow_blocks<TS>()
 // decision before that step's first store.
 constexpr int MULTI_THREADS = 256;
 
-template <typename TS, typename TC, int TRACE, bool ONE>
+template <typename TS, typename TC, bool ONE>
 __global__ void __launch_bounds__(MULTI_THREADS, 2)
     k_flow_multi(TS* f, TS* link, const SparseView S, const FlowParams P, Tracer* tr, double* partials, GridSync* gs, int steps,
                  int odd, int64_t k_west_end, int64_t k_east_begin, int* err) {
     __shared__ double sh[32];
-    __shared__ double ring[TRACE ? TRACER_WINDOW : 1];
+    __shared__ double ring[TRACER_WINDOW];
     __shared__ int s_conv;  // the tracer's decision: set once, before the step after the one it settles
-    if (TRACE && tr->converged) return;  // a batch continues past convergence as no-ops
+    if (tr->converged) return;  // a batch continues past convergence as no-ops
     const int tid = threadIdx.x;
     if (tid == 0) s_conv = 0;
     const int64_t k = (int64_t)blockIdx.x * MULTI_THREADS + tid, stride = (int64_t)gridDim.x * MULTI_THREADS;
@@ -482,15 +482,11 @@ __global__ void __launch_bounds__(MULTI_THREADS, 2)
     const bool bgk = live && P.dyn[code] == DYN_BGK;
     const int side = k < k_west_end ? -1 : (k >= k_east_begin ? 1 : 0);
     const TC rho = (TC)((side < 0 ? P.rho_w : P.rho_e) - 1.0), omega = (TC)P.omega[code];
-    int head = 0, count = 0;
-    if (TRACE) {
-        for (int q = tid; q < TRACER_WINDOW; q += MULTI_THREADS) ring[q] = tr->ring[q];
-        head = tr->head;
-        count = tr->count;
-    }
+    for (int q = tid; q < TRACER_WINDOW; q += MULTI_THREADS) ring[q] = tr->ring[q];
+    int head = tr->head, count = tr->count;
     double energy = 0;
-    // the stored average energy of step `n` (1, 2, ...) from the blocks' sums; with TRACE the tracer's
-    // window and its criterion. By warp 0 alone, while the other warps collide.
+    // the stored average energy of step `n` (1, 2, ...) from the blocks' sums, the tracer's window and its
+    // criterion. By warp 0 alone, while the other warps collide.
     auto warp_total = [](double v) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -502,7 +498,6 @@ __global__ void __launch_bounds__(MULTI_THREADS, 2)
         for (int q = tid; q < (int)gridDim.x; q += 32) v += __ldcg(part + q);
         v = warp_total(v);
         energy = P.n_bgk > 0 ? 0.5 * v / (double)P.n_bgk : 0.0;
-        if (!TRACE) return;
         if (tid == 0) ring[head] = energy;
         __syncwarp();
         head = (head + 1) % TRACER_WINDOW;
@@ -537,17 +532,15 @@ __global__ void __launch_bounds__(MULTI_THREADS, 2)
                 }
             }
         }
-        if (TRACE && done > 0 && tid < 32) trace(done);
+        if (done > 0 && tid < 32) trace(done);
         double e = 0;
         if (bgk) {
             if (side < 0) regularize19<TC>(g, -1, rho);
             else if (side > 0) regularize19<TC>(g, 1, rho);
             e = (double)bgk19<TC>(g, omega);
         }
-        if (TRACE) {
-            __syncthreads();
-            if (s_conv) break;
-        }
+        __syncthreads();
+        if (s_conv) break;
         if (live) {
             if (odd_step) {
 #pragma unroll
@@ -570,10 +563,8 @@ __global__ void __launch_bounds__(MULTI_THREADS, 2)
             }
         }
         ++done;
-        if (TRACE || done == steps) {  // without the tracer only the last step's energy is stored
-            const double bt = block_sum(e, sh);
-            if (tid == 0) partials[(done & 1) * gridDim.x + blockIdx.x] = bt;
-        }
+        const double bt = block_sum(e, sh);
+        if (tid == 0) partials[(done & 1) * gridDim.x + blockIdx.x] = bt;
         if (!(ok = grid_barrier(gs, (unsigned)done))) break;
     }
     if (!ok) {
@@ -584,16 +575,13 @@ __global__ void __launch_bounds__(MULTI_THREADS, 2)
     __syncthreads();
     if (tid < 32 && !s_conv) trace(done);
     __syncthreads();
-    if (TRACE)
-        for (int q = tid; q < TRACER_WINDOW; q += MULTI_THREADS) tr->ring[q] = ring[q];
+    for (int q = tid; q < TRACER_WINDOW; q += MULTI_THREADS) tr->ring[q] = ring[q];
     if (tid == 0) {
         tr->energy = energy;
         tr->iterations += done;
-        if (TRACE) {
-            tr->head = head;
-            tr->count = count;
-            if (s_conv) tr->converged = 1;
-        }
+        tr->head = head;
+        tr->count = count;
+        if (s_conv) tr->converged = 1;
     }
 }
 
@@ -834,17 +822,18 @@ static int flow_gather_grid(clb_handle* h) {
 }
 
 // Blocks of k_flow_multi for this lattice, 0 where a launch per step is faster; h->flow_multi_one: every
-// node has a resident thread. us per step, one launch per step -> many steps per launch, by nodes:
-//   11 k: FP64 8.8 -> 4.0, FP32 8.2 -> 3.1, FP16 9.2 -> 3.2;   27 k: 8.8 -> 4.2, 8.2 -> 3.2, 9.2 -> 3.3;
-//   91 k (walked): 13.3 -> 9.1, 10.8 -> 7.4, 12.3 -> 8.4;      214 k: 19.4 -> 14.7, 15.0 -> 11.4, 18.1 -> 13.3;
-//   482 k: 35.9 -> 30.6, 22.5 -> 22.7, 27.9 -> 25.5;           1067 k: 81 -> 79, 45 -> 52, 53 -> 51.
+// node has a resident thread. us per traced step, one launch per step -> many steps per launch, by nodes:
+//   11 k: FP64 13.5 -> 9.2, FP32 10.4 -> 4.8, FP16 12.6 -> 5.7;  91 k (walked): 17.0 -> 12.6, 13.4 -> 10.8, 17.9 -> 11.7;
+//   214 k: 23.2 -> 17.7, 17.0 -> 14.2, 22.3 -> 16.1;             482 k: 35.9 -> 37.5, 22.5 -> 24.6, 27.9 -> 27.7.
+// Steps without the tracer need no grid-wide sum and go one to a chained launch at every size (many steps per
+// launch: 27 k nodes FP32 3.2 against 2.95, 91 k 7.3 against 4.9, 214 k FP64 14.7 against 12.0).
 constexpr int64_t MULTI_MAX_NODES = 400000;
 
 template <typename TS, typename TC>
 static int flow_multi_blocks(clb_handle* h) {
     int one = 0, loop = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&one, k_flow_multi<TS, TC, 1, true>, MULTI_THREADS, 0) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&loop, k_flow_multi<TS, TC, 1, false>, MULTI_THREADS, 0) != cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&one, k_flow_multi<TS, TC, true>, MULTI_THREADS, 0) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&loop, k_flow_multi<TS, TC, false>, MULTI_THREADS, 0) != cudaSuccess)
         return 0;
     const int64_t need = (h->flow_sp.K + MULTI_THREADS - 1) / MULTI_THREADS;
     h->flow_multi_one = need <= (int64_t)one * h->num_sms;
@@ -1070,7 +1059,7 @@ static void launch_flow(clb_handle* h, bool odd, int trace, int count, bool afte
 }
 
 template <typename TS, typename TC>
-static cudaError_t launch_flow_multi(clb_handle* h, int n, bool trace) {
+static cudaError_t launch_flow_multi(clb_handle* h, int n) {
     GridSync* gs = (GridSync*)(h->d_err + 2);
     cudaError_t e = cudaMemsetAsync(gs, 0, sizeof(GridSync), h->stream);
     if (e != cudaSuccess) return e;
@@ -1081,25 +1070,25 @@ static cudaError_t launch_flow_multi(clb_handle* h, int n, bool trace) {
                     &h->d_err};
     ++h->launches;
     const void* kern = h->flow_multi_one
-                           ? (trace ? (const void*)k_flow_multi<TS, TC, 1, true> : (const void*)k_flow_multi<TS, TC, 0, true>)
-                           : (trace ? (const void*)k_flow_multi<TS, TC, 1, false> : (const void*)k_flow_multi<TS, TC, 0, false>);
+                           ? (const void*)k_flow_multi<TS, TC, true>
+                           : (const void*)k_flow_multi<TS, TC, false>;
     return cudaLaunchCooperativeKernel(kern, dim3(h->flow_multi), dim3(MULTI_THREADS), args, 0, h->stream);
 }
 
-// A small lattice takes its steps in launches of up to MULTI_STEPS (k_flow_multi); a call of one or two
-// steps, and every other lattice, a launch per step.
+// A small lattice takes its traced steps in launches of up to MULTI_STEPS (k_flow_multi); a call of one or
+// two of them, steps without the tracer, and every other lattice, a launch per step.
 constexpr int MULTI_STEPS = 1024, MULTI_MIN_STEPS = 3;
 
 clb_status flow_step(clb_handle* h, int n, bool trace, double eps) {
     (void)eps;
-    if (h->flow_multi && !h->flow_tuned && n >= MULTI_MIN_STEPS) {
+    if (trace && h->flow_multi && !h->flow_tuned && n >= MULTI_MIN_STEPS) {
         for (int k = 0; k < n; k += MULTI_STEPS) {
             const int m = std::min(MULTI_STEPS, n - k);
             cudaError_t e;
             switch (h->flow_prec) {
-                case CLB_F64: e = launch_flow_multi<double, double>(h, m, trace); break;
-                case CLB_F32: e = launch_flow_multi<float, float>(h, m, trace); break;
-                default: e = launch_flow_multi<__half, float>(h, m, trace); break;
+                case CLB_F64: e = launch_flow_multi<double, double>(h, m); break;
+                case CLB_F32: e = launch_flow_multi<float, float>(h, m); break;
+                default: e = launch_flow_multi<__half, float>(h, m); break;
             }
             if (e != cudaSuccess) return cuda_check(h, e, "flow steps");
             h->flow_iters += m;
@@ -1367,10 +1356,9 @@ clb_status flow_autotune(clb_handle* h, int steps, char* report, int report_len)
     };
     h->flow_tuned = false;
     const float base = timed();
-    const char* base_name = h->flow_multi && steps >= MULTI_MIN_STEPS ? "multi" : "stream";
     {
         char buf[64];
-        snprintf(buf, sizeof(buf), "%s:%.1fus", base_name, 1e3f * base / steps);
+        snprintf(buf, sizeof(buf), "stream:%.1fus", 1e3f * base / steps);
         rep += buf;
     }
     h->flow_tuned = true;
@@ -1404,7 +1392,7 @@ clb_status flow_autotune(clb_handle* h, int steps, char* report, int report_len)
     cudaFree(sl);
     h->flow_iters = iters0;
     char buf[64];
-    if (!h->flow_tuned) snprintf(buf, sizeof(buf), " -> %s", base_name);
+    if (!h->flow_tuned) snprintf(buf, sizeof(buf), " -> stream");
     else if (best_pipe) snprintf(buf, sizeof(buf), " -> tma=%d,pipe", best_tma);
     else snprintf(buf, sizeof(buf), " -> tma=%d,minb=%d", best_tma, best_minb);
     rep += buf;
