@@ -793,8 +793,8 @@ class Batch:
         _check_global(lib().clb_batch_step(self.b, int(n), int(flow), int(transport)))
 
     def schedule(self, persistent=True, tile=2048, lag=8, steps_per_launch=2, ctas_per_sm=4, staged_flow=False):
-        """persistent: the item-table schedule; else one launch per lattice and step, the flow step
-        through the staged kernels when staged_flow (4- and 8-byte storage)."""
+        """persistent: the item-table schedule; else one launch per lattice and step (staged_flow
+        selects the same launches, 4- and 8-byte storage)."""
         mode = 1 if persistent else (2 if staged_flow else 0)
         _check_global(lib().clb_batch_schedule(self.b, mode, int(tile), int(lag), int(steps_per_launch),
                                                int(ctas_per_sm)))

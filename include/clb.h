@@ -159,24 +159,26 @@ clb_status clb_synchronize(clb_handle* h);
 clb_status clb_set_stream(clb_handle* h, void* stream);
 clb_status clb_get_stream(clb_handle* h, void** stream);
 
-/* Launch-shape and kernel-variant knobs (used by the autotuner; defaults are tuned for B200):
- *   "flow_even_tma"  1: even AA step through shared-memory tiles and bulk copies (default),
+/* Launch-shape and kernel-variant knobs (used by the autotuner). By default every flow and transport
+ * step is streamed (one node per thread, no staging; many steps per launch on small lattices where
+ * that is faster); setting any "flow_" key takes the flow steps through the kernels it names:
+ *   "flow_even_tma"  1: even AA step through shared-memory tiles and bulk copies,
  *                    0: the plain per-thread load/store step;
  *   "flow_min_blocks" 2 or 3: resident CTAs per SM the gather/scatter step is compiled for
  *                    (register budget 128 or 80 per thread); takes effect at clb_flow_init;
  *   "flow_odd_pipe"  1: odd AA step with the next node's gathers staged in shared memory by
- *                    asynchronous copies while a node is collided (default for FP64/FP32
- *                    storage; an error for FP16 storage, which always runs the plain step),
+ *                    asynchronous copies while a node is collided (FP64/FP32 storage;
+ *                    an error for FP16 storage, which always runs the plain step),
  *                    0: the plain step;
  *   "ade_pipe"       1: transport step with the next node's gathers staged in shared memory by
  *                    asynchronous copies while a node is finished (used for FP64/FP32 storage
  *                    where two slot sets per thread leave two resident CTAs per SM, i.e. up to
- *                    8 FP32 or 4 FP64 species), 0: the plain step (default: fewer resident
- *                    warps made the pipelined step slower on B200).
+ *                    8 FP32 or 4 FP64 species), 0: the streamed step (default), or where an
+ *                    abiotic law, a gate or a rate-law file couples the species the staged one.
  * Unknown keys are an error. */
 clb_status clb_tune(clb_handle* h, const char* key, int value);
 
-/* Times every kernel variant of the flow step over `steps` steps on this domain and keeps the
+/* Times the default and every kernel variant of the flow step over `steps` steps on this domain and keeps the
  * fastest; the lattice state is saved and restored, so the simulation is unchanged. A one-line
  * report of the timings is written to `report` (may be NULL). */
 clb_status clb_autotune(clb_handle* h, int steps, char* report, int report_len);
@@ -555,9 +557,8 @@ clb_status clb_batch_autotune(clb_batch* batch, int steps, char* report, int rep
  * `lag` >= 1 domains between a domain's successive steps in the item table, an even 2..8 steps
  * per launch, and registers budgeted for `ctas_per_sm` resident CTAs per SM (4 always; 6 and 8
  * for FP32 / FP16 storage with up to 4 mobile species); persistent == 0: one launch per lattice
- * and step (the other arguments are ignored); persistent == 2: the same with the flow step
- * through the staged kernels (bulk-copied tiles on even steps, the next node's gathers in flight
- * on odd steps; FP32 / FP64 flow storage). The persistent schedule needs one storage type for
+ * and step (the other arguments are ignored); persistent == 2: the same launches (accepted for
+ * FP32 / FP64 flow storage, reported back as 2). The persistent schedule needs one storage type for
  * flow and transport. clb_batch_get_schedule reports the same three values. */
 clb_status clb_batch_schedule(clb_batch* batch, int persistent, int tile, int lag, int steps_per_launch,
                               int ctas_per_sm);
