@@ -363,8 +363,9 @@ __device__ __forceinline__ TC gather_flow(const TS* p) {
 // The stored average energy of a streamed step from its warps' sums, and the tracer (a launch after the
 // step's: inside it, a barrier, a fence and a counter per 128-node block cost the FP32 256^3 pack 125 us of a
 // 226 us step).
-__global__ void __launch_bounds__(256) k_flow_energy(const double* __restrict__ warp_sums, int64_t n, Tracer* tr, double* partials,
+__global__ void __launch_bounds__(256) k_flow_energy(const double* warp_sums, int64_t n, Tracer* tr, double* partials,
                                                      int64_t n_bgk, int trace, int count) {
+    step_wait();
     if (trace && tr->converged) return;
     __shared__ double sh[32];
     double v = 0;
@@ -384,10 +385,10 @@ __global__ void __launch_bounds__(256) k_flow_energy(const double* __restrict__ 
 // (8.7 M) FP32 316 -> 292 (4.2 -> 4.6 TB/s of algorithmic traffic); 199x143x131 (1.4 M) FP64 103 -> 83 (5.3
 // TB/s), FP16 71 -> 37. Two to sixteen nodes per thread with the next one's metadata prefetched: 54 to 65
 // us instead of 52.4.
-// The node's |u|^2 where it is a BGK node, else 0; `settled`: nothing is stored.
+// The node's |u|^2 where it is a BGK node, else 0; nothing is stored where *converged is set.
 template <typename TS, typename TC, bool ODD>
 __device__ __forceinline__ double flow_stream_node(TS* __restrict__ f, const SparseView& S, const FlowParams& P, int64_t k,
-                                                   int64_t k_west_end, int64_t k_east_begin, int settled) {
+                                                   int64_t k_west_end, int64_t k_east_begin, const int* converged) {
     const uint32_t K32 = (uint32_t)S.KS;
     const FlowMeta M = flow_meta<ODD>(S, k);
     uint32_t off[19];
@@ -407,6 +408,9 @@ __device__ __forceinline__ double flow_stream_node(TS* __restrict__ f, const Spa
     }
     const int dyn = P.dyn[M.code];
     step_wait();
+    // a batch continues past convergence as no-ops: used before the stores only, so the load is not a
+    // round trip of its own
+    const int settled = converged ? *(volatile const int*)converged : 0;
     if (dyn == DYN_BB) return 0.0;  // a stored bounce-back node: the identity on AA slots
     double e = 0;
     TC g[19];
@@ -426,14 +430,12 @@ __device__ __forceinline__ double flow_stream_node(TS* __restrict__ f, const Spa
 
 template <typename TS, typename TC, bool ODD, bool ENERGY>
 __global__ void __launch_bounds__(STREAM_FLOW_THREADS, (stream_flow_blocks<TS>()))
-    k_flow_stream(TS* __restrict__ f, const SparseView S, const FlowParams P, const Tracer* __restrict__ tr,
+    k_flow_stream(TS* __restrict__ f, const SparseView S, const FlowParams P, const Tracer* tr,
                   double* __restrict__ warp_sums, int trace, int64_t k_west_end, int64_t k_east_begin) {
-    // a batch continues past convergence as no-ops: looked at before the stores only, so the load is not a
-    // round trip of its own
-    const int settled = ENERGY && trace ? tr->converged : 0;
+    const int* converged = ENERGY && trace ? &tr->converged : nullptr;
     const int64_t k = (int64_t)blockIdx.x * STREAM_FLOW_THREADS + threadIdx.x;
     if (k >= S.K) step_wait();
-    double e = k < S.K ? flow_stream_node<TS, TC, ODD>(f, S, P, k, k_west_end, k_east_begin, settled) : 0.0;
+    double e = k < S.K ? flow_stream_node<TS, TC, ODD>(f, S, P, k, k_west_end, k_east_begin, converged) : 0.0;
     if (ENERGY) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
@@ -601,7 +603,7 @@ __global__ void __launch_bounds__(STREAM_FLOW_THREADS, (stream_flow_blocks<TS>()
     __syncthreads();
     const BatchDomain& D = *reinterpret_cast<const BatchDomain*>(words);  // its members before g only
     for (int i = threadIdx.x; i < T.count; i += STREAM_FLOW_THREADS)
-        flow_stream_node<TS, TC, ODD>((TS*)D.f, D.fs, D.fp, T.first + i, D.fkw, D.fke, 0);
+        flow_stream_node<TS, TC, ODD>((TS*)D.f, D.fs, D.fp, T.first + i, D.fkw, D.fke, nullptr);
 }
 
 void launch_flow_batch(const BatchView& B, int prec, bool odd, cudaStream_t st) {
@@ -975,13 +977,10 @@ clb_status flow_init(clb_handle* h, double delta_p) {
     return cuda_check(h, cudaGetLastError(), "flow init");
 }
 
-// The streamed step, except where a tuning key selects the tiled and pipelined kernels and for a traced FP32
-// step: those form the energy in the step itself, where the streamed one needs a launch after it (482 k
-// nodes FP32 22.3 us per traced step against 24.9, 2.6 M 70 against 73, 6.8 M 251 against 258; FP64 35.1
-// against 34.2, 119 against 111, 455 against 421).
-static bool flow_streams(const clb_handle* h, bool trace) {
-    return !h->flow_tuned && !(trace && h->flow_prec == CLB_F32);
-}
+// The streamed step, except where a tuning key selects the tiled and pipelined kernels. A traced step is two
+// chained launches, the step and its energy (tiled and pipelined kernels -> streamed, us per traced step: 480 k
+// nodes FP32 23.1 -> 22.4, 1.3 M 55.5 -> 54.5, 3.8 M 153.6 -> 147.4; FP64 3.8 M 261 -> 237, FP16 174 -> 124).
+static bool flow_streams(const clb_handle* h) { return !h->flow_tuned; }
 
 // One step. The streamed step forms the stored energy, and counts `count` iterations, only where count is
 // not 0; the kernels a tuning key selects do both at every step.
@@ -990,7 +989,7 @@ static void launch_flow(clb_handle* h, bool odd, int trace, int count, bool afte
     const FlowParams& P = h->fp;
     const SparseView S = view_of(h->flow_sp);
     const int grid = h->flow_grid;
-    if (flow_streams(h, trace)) {
+    if (flow_streams(h)) {
         const unsigned g = (unsigned)std::max<int64_t>(1, flow_tiles(h));
         auto go = [&](auto kern, auto* ts) {
             using TS = std::remove_pointer_t<decltype(ts)>;
@@ -1008,8 +1007,8 @@ static void launch_flow(clb_handle* h, bool odd, int trace, int count, bool afte
 #undef CLB_STREAM
         if (count) {
             ++h->launches;
-            k_flow_energy<<<h->num_sms, 256, 0, h->stream>>>(h->d_partials + h->partial_cap, (int64_t)g * (STREAM_FLOW_THREADS / 32),
-                                                             h->d_tracer, h->d_partials, P.n_bgk, trace, count);
+            launch_step(true, k_flow_energy, h->num_sms, 256, 0, h->stream, h->d_partials + h->partial_cap,
+                        (int64_t)g * (STREAM_FLOW_THREADS / 32), h->d_tracer, h->d_partials, P.n_bgk, trace, count);
         }
         return;
     }
@@ -1096,7 +1095,7 @@ clb_status flow_step(clb_handle* h, int n, bool trace, double eps) {
         return CLB_OK;
     }
     for (int k = 0; k < n; ++k) {
-        launch_flow(h, (h->flow_iters & 1) != 0, trace ? 1 : 0, trace ? 1 : (k + 1 == n ? n : 0), k > 0 && !trace && flow_streams(h, false));
+        launch_flow(h, (h->flow_iters & 1) != 0, trace ? 1 : 0, trace ? 1 : (k + 1 == n ? n : 0), k > 0 && flow_streams(h));
         h->flow_iters += 1;
     }
     return cuda_check(h, cudaGetLastError(), "flow step");
@@ -1127,7 +1126,7 @@ clb_status flow_solve(clb_handle* h, int max_it, double eps, int* iterations, bo
     // decision before its stores, which saves every other step a round trip), so the run up to a full
     // window goes at once and then few at a time: the wait costs about 15 us, a step of a lattice that
     // takes the streamed kernel 16 us and more. The other kernels return at once.
-    const bool multi = h->flow_multi && !h->flow_tuned, stream = !multi && flow_streams(h, true);
+    const bool multi = h->flow_multi && !h->flow_tuned, stream = !multi && flow_streams(h);
     int chunk = multi ? MULTI_STEPS : stream ? std::max(4, TRACER_WINDOW - t0.count) : 64;
     bool conv = false;
     while (done < max_it) {
