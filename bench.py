@@ -744,7 +744,7 @@ def main():
     per_launch = ms_transport / max(1, iters)
     achieved = alg_node * n_open / (per_launch * 1e-3) / 1e9
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-            "traffic": traffic_per_launch("k_ade_aa_f32_pack256cube_8species"), "peak_source": peak_kind,
+            "traffic": traffic_per_launch("k_ade_stream_f32_pack256cube_8species"), "peak_source": peak_kind,
             "algorithmic_bytes_per_launch": alg_node * n_open, "algorithmic_bytes_per_node": alg_node,
             "biomass_flagged_fraction": [bio_start[1], bio_end[1]],
             "kernel": "k_ade_stream (all 8 species fused, even/odd AA steps) + k_neumann, the fused transport "
