@@ -189,7 +189,8 @@ __device__ __forceinline__ void ade_collide_store(TS* f, const uint32_t (&off)[7
 //     are added to the stored populations afterwards. A stored 4- or 8-byte population is the
 //     collision's own value, so the sum is rounded as if the deposit had been added before the
 //     store, and only the nodes with biomass (a few per cent) pay for the coupling.
-//   dual ahead: dual Monod otherwise; the coupled densities are read once more ahead of the step.
+//   dual ahead: dual Monod otherwise (immobile partners, 2-byte storage); the coupled densities are read once
+//     more ahead of the step.
 enum StreamLaw { STREAM_NONE, STREAM_SEPARABLE, STREAM_DUAL_AFTER, STREAM_DUAL_AHEAD };
 constexpr int STREAM_MICROBES = 2;  // of "dual after"
 
@@ -358,6 +359,15 @@ __device__ __forceinline__ void ade_stream_species(TS* g, double* imm, double* b
             }
             ade_collide_store<TS, TC>(g + (int64_t)s * S.SS, off, q[v], r, wk[s], d, A.ux, A.uy, A.uz, P.S == 1);
         }
+    }
+    if (LAW == STREAM_DUAL_AHEAD && nm == 0 && hb) {
+        // no species is mobile: there was no group to take the coupled laws with
+        dual_monod<TC>(
+            P, bio, nd, [](int, const double* p) { return *p; },
+            [&](int s) { return floored<TC>((TC)imm[(int64_t)s * P.N + nd]); },
+            [&](int s, TC d) {
+                if (d != (TC)0) imm[(int64_t)s * P.N + nd] += (double)d;
+            });
     }
     if (LAW == STREAM_DUAL_AFTER && hb) {
         cp_async_wait_all();  // each thread reads only its own slots
