@@ -74,26 +74,6 @@ inline AdeStep<TC> ade_step_params(const AdeParams& P, int n_mobile) {
     return Q;
 }
 
-// A gather that keeps its place in program order: the compiler would otherwise sink a group's later
-// gathers below the first species' arithmetic to save registers, and the loads would no longer be
-// in flight together.
-template <typename TS, typename TC>
-__device__ __forceinline__ TC gather(const TS* p) {
-    if constexpr (sizeof(TS) == 8) {
-        double v;
-        asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
-        return (TC)v;
-    } else if constexpr (sizeof(TS) == 4) {
-        float v;
-        asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
-        return (TC)v;
-    } else {
-        unsigned short v;
-        asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
-        return (TC)(__half2float(__ushort_as_half(v)) * HALF_INV);
-    }
-}
-
 // One domain of a batch as the streamed step sees it (device copy, one per domain).
 template <typename TC>
 struct StreamDomain {

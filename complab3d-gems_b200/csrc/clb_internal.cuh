@@ -64,6 +64,25 @@ template <typename TS>
 __device__ __forceinline__ double ldd(const TS* p) { return (double)(*p); }
 template <>
 __device__ __forceinline__ double ldd<__half>(const __half* p) { return (double)(__half2float(*p) * HALF_INV); }
+// ld() that keeps its place in program order: the compiler would otherwise sink a node's later gathers below
+// the first ones' arithmetic to save registers, and the loads would no longer be in flight together. The
+// clobber orders it against the node's stores to the same slots and against barriers and waits.
+template <typename TS, typename TC>
+__device__ __forceinline__ TC gather(const TS* p) {
+    if constexpr (sizeof(TS) == 8) {
+        double v;
+        asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+        return (TC)v;
+    } else if constexpr (sizeof(TS) == 4) {
+        float v;
+        asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+        return (TC)v;
+    } else {
+        unsigned short v;
+        asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p) : "memory");
+        return (TC)(__half2float(__ushort_as_half(v)) * HALF_INV);
+    }
+}
 template <typename TS, typename TC>
 __device__ __forceinline__ void st(TS* p, TC v) { *p = (TS)v; }
 template <>

@@ -342,24 +342,6 @@ constexpr int STREAM_FLOW_THREADS = 128;
 template <typename TS>
 constexpr int stream_flow_blocks() { return sizeof(TS) == 4 ? 6 : 5; }
 
-// A gather that keeps its place in program order, so a node's gathers are in flight together.
-template <typename TS, typename TC>
-__device__ __forceinline__ TC gather_flow(const TS* p) {
-    if constexpr (sizeof(TS) == 8) {
-        double v;
-        asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
-        return (TC)v;
-    } else if constexpr (sizeof(TS) == 4) {
-        float v;
-        asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
-        return (TC)v;
-    } else {
-        unsigned short v;
-        asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
-        return (TC)(__half2float(__ushort_as_half(v)) * HALF_INV);
-    }
-}
-
 // The stored average energy of a streamed step from its warps' sums, and the tracer (a launch after the
 // step's: inside it, a barrier, a fence and a counter per 128-node block cost the FP32 256^3 pack 125 us of a
 // 226 us step).
@@ -415,7 +397,7 @@ __device__ __forceinline__ double flow_stream_node(TS* __restrict__ f, const Spa
     double e = 0;
     TC g[19];
 #pragma unroll
-    for (int i = 0; i < 19; ++i) g[i] = gather_flow<TS, TC>(f + off[i]);
+    for (int i = 0; i < 19; ++i) g[i] = gather<TS, TC>(f + off[i]);
     if (dyn == DYN_BGK) {
         if (k < k_west_end) regularize19<TC>(g, -1, (TC)(P.rho_w - 1.0));
         else if (k >= k_east_begin) regularize19<TC>(g, 1, (TC)(P.rho_e - 1.0));
