@@ -24,6 +24,7 @@
 // (3*sizeof(arith)) and the material byte shared by all species.
 #include "batch.cuh"
 #include "flow_node.cuh"
+#include "grid_sync.cuh"
 #include "kinetics.cuh"
 #include "tma.cuh"
 
@@ -994,13 +995,13 @@ clb_status ade_init(clb_handle* h, const clb_species_desc* sp, int S) {
     if ((e = cudaMalloc(&h->d_u, usize(h->ade_prec) * 3 * K1)) != cudaSuccess) return cuda_check(h, e, "velocity");
     if ((e = cudaMalloc(&h->d_neu, sizeof(double) * S * 2 * h->g.plane + sizeof(int) * 16)) != cudaSuccess)
         return cuda_check(h, e, "boundary store");
-    if ((e = cudaMalloc(&h->d_sync, 4 * sizeof(int))) != cudaSuccess) return cuda_check(h, e, "barrier");
-    cudaMemsetAsync(h->d_sync, 0, 4 * sizeof(int), h->stream);
+    if ((e = cudaMalloc(&h->d_sync, sizeof(GridSync))) != cudaSuccess) return cuda_check(h, e, "barrier");
+    cudaMemsetAsync(h->d_sync, 0, sizeof(GridSync), h->stream);
     if (!h->h_flags) {
         // host-mapped flags the transport step sets (read by the host without a copy)
-        if ((e = cudaHostAlloc((void**)&h->h_flags, 16, cudaHostAllocMapped)) != cudaSuccess)
+        if ((e = cudaHostAlloc((void**)&h->h_flags, sizeof(int) * FLAG_COUNT, cudaHostAllocMapped)) != cudaSuccess)
             return cuda_check(h, e, "status flags");
-        std::memset(h->h_flags, 0, 16);
+        std::memset(h->h_flags, 0, sizeof(int) * FLAG_COUNT);
         if ((e = cudaHostGetDevicePointer((void**)&h->d_flags, h->h_flags, 0)) != cudaSuccess)
             return cuda_check(h, e, "status flags");
     }
@@ -1047,8 +1048,9 @@ clb_status ade_init(clb_handle* h, const clb_species_desc* sp, int S) {
     h->ade_iters = 0;
     h->neu_iter = -1;
     h->ade_grid = h->num_sms * 4;
-    P.nonfinite = h->d_flags;
-    if (h->h_flags) h->h_flags[0] = 0;
+    P.nonfinite = h->d_flags + FLAG_NONFINITE;
+    cudaStreamSynchronize(h->stream);  // no step in flight may set a flag after the clear
+    std::memset(h->h_flags, 0, sizeof(int) * FLAG_COUNT);
     h->ade_ready = true;
     return cuda_check(h, cudaGetLastError(), "ade init");
 }
@@ -1542,7 +1544,7 @@ void ade_refresh_neumann(clb_handle* h) { refresh_neumann(h); }
 // (complab.cpp:2796, 3116-3117): the next clb_ade_step, and clb_synchronize once that step has
 // completed, return CLB_NONFINITE. Setting a species' populations clears the flag.
 clb_status ade_nonfinite_check(clb_handle* h) {
-    if (h->h_flags && ((volatile int*)h->h_flags)[0])
+    if (h->h_flags && ((volatile int*)h->h_flags)[FLAG_NONFINITE])
         return fail(h, CLB_NONFINITE, "a transport step met a non-finite (NaN or Inf) concentration");
     return CLB_OK;
 }
@@ -1550,6 +1552,8 @@ clb_status ade_nonfinite_check(clb_handle* h) {
 clb_status ade_step(clb_handle* h, int n) {
     if (!h->ade_ready) return fail(h, CLB_NOT_INITIALIZED, "clb_ade_init first");
     if (h->M > 0 && h->d_bio == nullptr) return fail(h, CLB_INVALID_ARG, "biomass missing");
+    const clb_status ws = waits_check(h, false, true);
+    if (ws != CLB_OK) return ws;
     if (ade_nonfinite_check(h) != CLB_OK) return CLB_NONFINITE;
     if (ade_streams(h->ap) && !h->ade_pipe && h->spec_mode == CLB_SPEC_OFF) {
         refresh_neumann(h);  // the values of face nodes whose inner neighbour is no fluid node
@@ -1587,6 +1591,8 @@ clb_status ade_step(clb_handle* h, int n) {
 clb_status ade_couple(clb_handle* h) {
     if (!h->ade_ready) return fail(h, CLB_NOT_INITIALIZED, "clb_ade_init first");
     if (!h->flow_ready) return fail(h, CLB_NOT_INITIALIZED, "clb_flow_init first");
+    const clb_status ws = waits_check(h, true, false);
+    if (ws != CLB_OK) return ws;
     return flow_velocity_at(h, h->ade_sp.node, h->ade_sp.K, h->d_u, h->ade_sp.K, h->ade_prec == CLB_F64 ? 0 : 1);
 }
 
@@ -1623,7 +1629,7 @@ clb_status ade_set_populations(clb_handle* h, int s, const double* host, int shi
     if (s < 0 || s >= h->S) return fail(h, CLB_INVALID_ARG, "species index out of range");
     if (h->h_flags) {
         cudaStreamSynchronize(h->stream);  // no step in flight may set the flag after the clear
-        h->h_flags[0] = 0;
+        h->h_flags[FLAG_NONFINITE] = 0;
     }
     s = h->u2i[s];
     if (h->ap.slot[s] < 0) return fail(h, CLB_INVALID_ARG, "not a mobile species");

@@ -168,7 +168,7 @@ constexpr int STREAM_MULTI_THREADS = 256;
 template <typename TS, typename TC, int U, int LAW>
 __global__ void __launch_bounds__(STREAM_MULTI_THREADS, 2)
     k_ade_stream_multi(TS* g, double* imm, double* bio, const TC* u, const SparseView S, const double* neu, const AdeStep<TC> P,
-                       int64_t kw, int64_t ke, int neumann, int steps, int odd, GridSync* gs, int* err) {
+                       int64_t kw, int64_t ke, int neumann, int steps, int odd, GridSync* gs, uint32_t polls, int* gave_up) {
     extern __shared__ __align__(16) unsigned char stream_smem[];
     constexpr int T = STREAM_MULTI_THREADS;
     struct Node {
@@ -214,6 +214,7 @@ __global__ void __launch_bounds__(STREAM_MULTI_THREADS, 2)
         if (odd_step) run(N.odd, I.odd);
         else run(N.even, I.even);
     };
+    if (*(volatile unsigned*)&gs->abort) return;  // a launch of the same call before this one gave up
     const int64_t k = (int64_t)blockIdx.x * T + threadIdx.x;
     Node N = {}, I = {};
     int64_t kp = -1;
@@ -232,8 +233,8 @@ __global__ void __launch_bounds__(STREAM_MULTI_THREADS, 2)
     for (int t = 0; t < steps; ++t) {
         const bool odd_step = ((odd + t) & 1) != 0;
         if (mine) step(k, N, kp, I, odd_step);
-        if (!grid_barrier(gs, (unsigned)t + 1)) {
-            if (threadIdx.x == 0) atomicExch(err, 1);
+        if (!grid_barrier(gs, (unsigned)t + 1, polls)) {
+            if (threadIdx.x == 0) *(volatile int*)gave_up = 1;
             return;
         }
     }
@@ -272,14 +273,15 @@ static bool launch_stream_multi_t(clb_handle* h, int steps, cudaError_t& e) {
         TS* g = (TS*)h->d_g;
         const TC* u = (const TC*)h->d_u;
         const double* neu = h->d_neu;
-        GridSync* gs = (GridSync*)(h->d_sync);
-        int* err = h->d_sync + 2;
+        GridSync* gs = (GridSync*)h->d_sync;
+        uint32_t polls = (uint32_t)h->barrier_polls;
+        int* gave_up = h->d_flags + FLAG_ADE_WAIT;
         int odd = (int)(h->ade_iters & 1);
         for (int t = 0; t < steps; t += STREAM_MULTI_STEPS, odd ^= STREAM_MULTI_STEPS & 1) {
             int n = std::min(STREAM_MULTI_STEPS, steps - t);
             void* args[] = {&g, &h->d_imm, &h->d_bio, &u, &S, &neu, &P, &h->ade_west_end, &h->ade_east_begin, &neumann, &n, &odd,
-                            &gs, &err};
-            if ((e = cudaMemsetAsync(gs, 0, sizeof(GridSync), h->stream)) != cudaSuccess) return true;
+                            &gs, &polls, &gave_up};
+            if ((e = cudaMemsetAsync(&gs->arrived, 0, sizeof(gs->arrived), h->stream)) != cudaSuccess) return true;
             ++h->launches;
             e = cudaLaunchCooperativeKernel((const void*)kern, dim3((unsigned)need), dim3(STREAM_MULTI_THREADS), args, sm, h->stream);
             if (e != cudaSuccess) return true;

@@ -26,6 +26,24 @@ clb_status cuda_check(clb_handle* h, cudaError_t e, const char* what) {
     return fail(h, e == cudaErrorMemoryAllocation ? CLB_OUT_OF_MEMORY : CLB_CUDA_ERROR, m);
 }
 
+clb_status waits_check(clb_handle* h, bool flow, bool ade, bool look) {
+    if (flow && look && h->flow_tuned && h->d_tracer) {
+        int gave_up = 0;
+        const cudaError_t e = copy_on_stream(h, &gave_up, &h->d_tracer->gave_up, sizeof(int), cudaMemcpyDeviceToHost);
+        if (e != cudaSuccess) return cuda_check(h, e, "tracer read");
+        if (gave_up) h->flow_gave_up = true;
+    }
+    if ((flow && h->flow_gave_up) || (ade && h->h_flags && ((volatile int*)h->h_flags)[FLAG_ADE_WAIT]))
+        return fail(h, CLB_TIMEOUT, "a bounded device wait gave up (a bulk copy or a grid-wide barrier did not complete); the "
+                                    "lattice is undefined until it is initialised again");
+    return CLB_OK;
+}
+
+// The status of a call that read a lattice back and waited for its stream: s, or that what it read is undefined.
+static clb_status readback(clb_handle* h, clb_status s, bool flow, bool ade) {
+    return s == CLB_OK ? waits_check(h, flow, ade, true) : s;
+}
+
 clb_status stage_rows(clb_handle* h, size_t per_voxel, int* rows) {
     const size_t row = per_voxel * (size_t)h->g.nz, all = per_voxel * (size_t)h->g.N;
     const size_t need = std::max(row, std::min(all, STAGE_BYTES));
@@ -127,7 +145,7 @@ clb_status clb_destroy(clb_handle* h) {
     cudaFree(h->d_mat);
     cudaFree(h->d_stage);
     cudaFree(h->d_mat_flow);
-    cudaFree(h->d_err);
+    cudaFree(h->d_flow_sync);
     cudaFree(h->d_spec_stats);
     cudaFree(h->d_mlp);
     cudaFree(h->d_mlp_bf16);
@@ -147,11 +165,7 @@ clb_status clb_synchronize(clb_handle* h) {
     CLB_ON_DEVICE(h);
     clb_status s = cuda_check(h, cudaStreamSynchronize(h->stream), "synchronize");
     if (s != CLB_OK) return s;
-    int flag = 0, flag2 = 0;
-    if (h->d_err) copy_on_stream(h, &flag, h->d_err, sizeof(int), cudaMemcpyDeviceToHost);
-    if (h->d_sync) copy_on_stream(h, &flag2, h->d_sync + 2, sizeof(int), cudaMemcpyDeviceToHost);
-    if (flag || flag2)
-        return fail(h, CLB_TIMEOUT, "a bounded device wait gave up (a bulk copy or a grid-wide barrier did not complete)");
+    if ((s = waits_check(h, true, true, true)) != CLB_OK) return s;
     return ade_nonfinite_check(h);
 }
 
@@ -188,6 +202,11 @@ clb_status clb_tune(clb_handle* h, const char* key, int value) {
     if (k == "flow_min_blocks") {
         if (value != 2 && value != 3) return fail(h, CLB_INVALID_ARG, "flow_min_blocks is 2 or 3");
         h->flow_minb = value;
+        return CLB_OK;
+    }
+    if (k == "barrier_polls") {
+        if (value < 0) return fail(h, CLB_INVALID_ARG, "barrier_polls must not be negative");
+        h->barrier_polls = value;
         return CLB_OK;
     }
     return fail(h, CLB_INVALID_ARG, "unknown tuning key '" + k + "'");
@@ -229,7 +248,7 @@ clb_status clb_flow_stats_get(clb_handle* h, double char_length, clb_flow_stats*
     if (!h || !out) return fail(h, CLB_INVALID_ARG, "null argument");
     CLB_ON_DEVICE(h);
     if (!h->flow_ready) return fail(h, CLB_NOT_INITIALIZED, "clb_flow_init first");
-    return flow_stats(h, char_length, out);
+    return readback(h, flow_stats(h, char_length, out), true, false);
 }
 
 clb_status clb_flow_solve_peclet(clb_handle* h, double peclet, double char_length, double tau_ade_fixed, int max_it,
@@ -348,7 +367,7 @@ clb_status clb_ade_step(clb_handle* h, int n) {
 clb_status clb_reduce(clb_handle* h, clb_stats* out) {
     if (!h || !out) return fail(h, CLB_INVALID_ARG, "null argument");
     CLB_ON_DEVICE(h);
-    return ade_reduce(h, out);
+    return readback(h, ade_reduce(h, out), false, true);
 }
 
 clb_status clb_set_abiotic_kinetics(clb_handle* h, int law, const double* params, int n_params, int surface_only) {
@@ -367,7 +386,7 @@ clb_status clb_precip_setup(clb_handle* h, const clb_precip_desc* desc) {
 clb_status clb_geometry_update(clb_handle* h, int* sealed, int* reopened) {
     if (!h) return fail(nullptr, CLB_INVALID_ARG, "null handle");
     CLB_ON_DEVICE(h);
-    return geometry_update(h, sealed, reopened);
+    return readback(h, geometry_update(h, sealed, reopened), true, true);
 }
 
 clb_status clb_ca_setup(clb_handle* h, const clb_ca_desc* desc) {
@@ -379,7 +398,7 @@ clb_status clb_ca_setup(clb_handle* h, const clb_ca_desc* desc) {
 clb_status clb_ca_step(clb_handle* h, int* sweeps, int* mask_changed) {
     if (!h) return fail(nullptr, CLB_INVALID_ARG, "null handle");
     CLB_ON_DEVICE(h);
-    return ca_step(h, sweeps, mask_changed);
+    return readback(h, ca_step(h, sweeps, mask_changed), false, true);
 }
 
 clb_status clb_refresh_dynamics(clb_handle* h, int species, int flow) {
@@ -443,7 +462,7 @@ clb_status clb_batch_destroy(clb_batch* batch) { return batch_destroy(batch); }
 clb_status clb_reduce_noalloc(clb_handle* h, clb_stats* out) {
     if (!h || !out) return fail(h, CLB_INVALID_ARG, "null argument");
     CLB_ON_DEVICE(h);
-    return ade_reduce_noalloc(h, out);
+    return readback(h, ade_reduce_noalloc(h, out), false, true);
 }
 
 clb_status clb_speciation_setup(clb_handle* h, const clb_speciation_desc* desc) {
@@ -527,16 +546,16 @@ clb_status clb_get_field(clb_handle* h, int field, int index, void* host, int dt
     if (field == CLB_FIELD_FLOW_VELOCITY) {
         if (dtype != 0 && dtype != 1) return fail(h, CLB_INVALID_ARG, "the flow velocity is read as float64 or float32");
         if (!h->flow_ready) return fail(h, CLB_NOT_INITIALIZED, "clb_flow_init first");
-        return flow_velocity(h, host, dtype, true);
+        return readback(h, flow_velocity(h, host, dtype, true), true, false);
     }
     if (dtype != 0) return fail(h, CLB_INVALID_ARG, "fields are read as float64");
     switch (field) {
         case CLB_FIELD_FLOW_POPULATIONS:
             if (!h->flow_ready) return fail(h, CLB_NOT_INITIALIZED, "clb_flow_init first");
-            return flow_populations(h, (double*)host);
-        case CLB_FIELD_CONCENTRATION: return ade_density(h, index, (double*)host);
-        case CLB_FIELD_ADE_POPULATIONS: return ade_populations(h, index, (double*)host);
-        case CLB_FIELD_BIOMASS: return ade_biomass(h, index, (double*)host);
+            return readback(h, flow_populations(h, (double*)host), true, false);
+        case CLB_FIELD_CONCENTRATION: return readback(h, ade_density(h, index, (double*)host), false, true);
+        case CLB_FIELD_ADE_POPULATIONS: return readback(h, ade_populations(h, index, (double*)host), false, true);
+        case CLB_FIELD_BIOMASS: return readback(h, ade_biomass(h, index, (double*)host), false, true);
         case CLB_FIELD_ADE_VELOCITY: return ade_velocity(h, (double*)host);
         case CLB_FIELD_CA_TOTAL: return ca_fields(h, 0, (double*)host);
         case CLB_FIELD_CA_AGE: return ca_fields(h, 1, (double*)host);

@@ -402,6 +402,7 @@ clb_status batch_step(clb_batch* b, int n, int flow_on, int ade_on) {
             return bfail(b, CLB_INVALID_ARG, "batched domains must be at the same step parity");
         cudaError_t e = cudaStreamSynchronize(h->stream);  // their own pending work first
         if (e != cudaSuccess) return bfail(b, CLB_CUDA_ERROR, std::string("batch step: ") + cudaGetErrorString(e));
+        if (waits_check(h, flow, ade, true) != CLB_OK) return bfail(b, CLB_TIMEOUT, "batch step: " + h->err);
     }
     if (b->persistent) {
         clb_status st = persist_steps(b, n, fodd, aodd, flow, ade);

@@ -110,6 +110,10 @@ clb_status clb_checkpoint_save(clb_handle* h, const char* path, int what) {
             ok = st == CLB_OK && put(f, buf.data(), sizeof(double) * buf.size());
         }
     }
+    if (ok) {
+        st = waits_check(h, (what & CLB_CKPT_FLOW) != 0, (what & CLB_CKPT_TRANSPORT) != 0, true);
+        ok = st == CLB_OK;
+    }
     if (ok && std::fflush(f) != 0) ok = false;
     if (std::fclose(f) != 0) ok = false;
     if (!ok || st != CLB_OK) {

@@ -129,7 +129,7 @@ struct Tracer {
     int32_t enabled;        // 1 while a solve runs
     int32_t converged;      // set once the criterion holds
     uint32_t done_blocks;   // completion counter of the running step
-    int32_t pad;
+    int32_t gave_up;        // set once a bounded wait of a step did: the lattice is undefined
 };
 
 // ------------------------------------------------------------------ flow parameters
@@ -268,10 +268,12 @@ struct clb_handle_s {
     bool flow_multi_one = false;      // its threads keep one node each
     bool flow_tuned = false;          // a per-step kernel variant was asked for (clb_tune) or measured faster
     int flow_pipe_grid = 0;           // its resident-CTA grid; 0 where it is not available
-    int* d_err = nullptr;             // device error flag (bounded waits that gave up)
+    int* d_flow_sync = nullptr;       // grid-wide barrier of the many-step flow launches (GridSync)
+    int barrier_polls = 1 << 24;      // limit of one wait at a grid-wide barrier (about 10 s); "barrier_polls"
     uint8_t* d_bflag = nullptr;       // [K] species-lattice nodes where biomass may act (AdeParams::bflag)
-    int* h_flags = nullptr;           // host-mapped pinned flags: [0] a transport step met a non-finite
-    int* d_flags = nullptr;           // density (its device alias)
+    bool flow_gave_up = false;        // a flow step's bounded wait did (the tracer's flag, seen by the host)
+    int* h_flags = nullptr;           // host-mapped pinned flags the transport steps set (enum AdeFlag)
+    int* d_flags = nullptr;           // their device alias
     int64_t flow_iters = 0;           // host mirror of the device iteration count
     double delta_p = 0;
 
@@ -290,7 +292,7 @@ struct clb_handle_s {
     double* d_imm = nullptr;          // [S][N] immobile concentrations (unused rows stay empty)
     double* d_bio = nullptr;          // [M][N] biomass
     void* d_u = nullptr;              // [3][K] advection velocity (arithmetic type)
-    int* d_sync = nullptr;            // [0], [1] grid-wide barrier of the many-step launches, [2] its wait gave up
+    int* d_sync = nullptr;            // grid-wide barrier of the many-step transport launches (GridSync)
     double* d_neu = nullptr;          // [S][2][ny*nz] stored boundary densities
     double* d_red = nullptr;          // scratch of clb_reduce (partials, then the result)
     void* d_stage = nullptr;          // staging of a field read back to the host (stage_rows)
@@ -364,6 +366,14 @@ struct clb_handle_s {
 namespace clb {
 // error helpers (api.cu)
 clb_status fail(clb_handle* h, clb_status s, const std::string& msg);
+// What a transport step tells the host without a copy, once its stream has been waited for: it met a non-finite
+// density; its wait at a grid-wide barrier gave up.
+enum AdeFlag { FLAG_NONFINITE, FLAG_ADE_WAIT, FLAG_COUNT };
+// CLB_TIMEOUT where a bounded wait of the flow (transport) step gave up, which leaves that lattice undefined
+// until clb_flow_init (clb_ade_init). Many flow steps to a launch are taken by flow_solve alone, which meets
+// the tracer's flag with its result (a pinned flag would cost clb_flow_init 2.5 ms); look: the stream has been
+// waited for and a step through tiles, which any call may have enqueued, is asked for with a copy.
+clb_status waits_check(clb_handle* h, bool flow, bool ade, bool look = false);
 // The handle's staging buffer of a readback, allocated on first use and kept (a cudaMalloc and cudaFree
 // per call took between 0.5 and 25 ms): at most STAGE_BYTES, or one row where a row is larger. *rows:
 // the rows of the box (nz voxels each) it holds at `per_voxel` bytes a voxel.

@@ -214,6 +214,7 @@ clb_status run(clb_handle* h, const clb_run_desc* d, clb_run_report* r) {
     r->launches = h->launches - launches0;
     if (st != CLB_OK) return st;
     if (e != cudaSuccess) return cuda_check(h, e, "run");
+    if ((st = waits_check(h, resolves, true)) != CLB_OK) return st;
     return ade_nonfinite_check(h);
 }
 

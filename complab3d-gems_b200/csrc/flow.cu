@@ -235,7 +235,7 @@ template <typename TS, typename TC>
 __global__ void __launch_bounds__(TILE, sizeof(TS) == 8 ? 2 : 4)
     k_flow_even_tma(TS* __restrict__ f, TS* __restrict__ link, const SparseView S, const FlowParams P,
                     Tracer* __restrict__ tr, double* __restrict__ partials, int trace, int64_t k_west_end,
-                    int64_t k_east_begin, int* __restrict__ err) {
+                    int64_t k_east_begin) {
     if (trace && tr->converged) return;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     TS* stages = reinterpret_cast<TS*>(smem_raw);
@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(TILE, sizeof(TS) == 8 ? 2 : 4)
             }
         }
         if (!mbar_wait(&full[q], (uint32_t)((j / NSTAGE) & 1))) {
-            if (tid == 0) { atomicExch(err, 1); s_abort = 1; }
+            if (tid == 0) { tr->gave_up = 1; s_abort = 1; }
         }
         __syncthreads();
         if (s_abort) break;
@@ -440,7 +440,7 @@ constexpr int MULTI_THREADS = 256;
 template <typename TS, typename TC, bool ONE>
 __global__ void __launch_bounds__(MULTI_THREADS, 2)
     k_flow_multi(TS* f, TS* link, const SparseView S, const FlowParams P, Tracer* tr, double* partials, GridSync* gs, int steps,
-                 int odd, int64_t k_west_end, int64_t k_east_begin, int* err) {
+                 int odd, int64_t k_west_end, int64_t k_east_begin, uint32_t polls) {
     __shared__ double sh[32];
     __shared__ double ring[TRACER_WINDOW];
     __shared__ int s_conv;  // the tracer's decision: set once, before the step after the one it settles
@@ -549,10 +549,10 @@ __global__ void __launch_bounds__(MULTI_THREADS, 2)
         ++done;
         const double bt = block_sum(e, sh);
         if (tid == 0) partials[(done & 1) * gridDim.x + blockIdx.x] = bt;
-        if (!(ok = grid_barrier(gs, (unsigned)done))) break;
+        if (!(ok = grid_barrier(gs, (unsigned)done, polls))) break;
     }
     if (!ok) {
-        if (tid == 0) atomicExch(err, 1);
+        if (tid == 0) tr->gave_up = 1;
         return;
     }
     if (blockIdx.x != 0) return;
@@ -936,11 +936,9 @@ clb_status flow_init(clb_handle* h, double delta_p) {
     const int64_t warps = std::max<int64_t>(1, flow_tiles(h)) * (STREAM_FLOW_THREADS / 32);
     if ((e = cudaMalloc(&h->d_partials, sizeof(double) * (pcap + warps))) != cudaSuccess) return cuda_check(h, e, "partials");
     h->partial_cap = pcap;
-    if (!h->d_err) {
-        // [0] the error flag; [2], [3] the grid-wide barrier of the many-step launches
-        if ((e = cudaMalloc(&h->d_err, 4 * sizeof(int))) != cudaSuccess) return cuda_check(h, e, "error flag");
-    }
-    cudaMemsetAsync(h->d_err, 0, 4 * sizeof(int), h->stream);
+    if (!h->d_flow_sync && (e = cudaMalloc(&h->d_flow_sync, sizeof(GridSync))) != cudaSuccess)
+        return cuda_check(h, e, "barrier");
+    h->flow_gave_up = false;
     switch (h->flow_prec) {
         case CLB_F64: h->flow_multi = flow_multi_blocks<double, double>(h); break;
         case CLB_F32: h->flow_multi = flow_multi_blocks<float, float>(h); break;
@@ -999,7 +997,7 @@ static void launch_flow(clb_handle* h, bool odd, int trace, int count, bool afte
 #define CLB_EVEN(TS, TC)                                                                                       \
         k_flow_even_tma<TS, TC><<<eg, TILE, even_smem<TS>(), h->stream>>>((TS*)h->d_f, (TS*)h->d_flink, S, P,  \
                                                                        h->d_tracer, h->d_partials, trace,     \
-                                                                       h->k_west_end, h->k_east_begin, h->d_err);
+                                                                       h->k_west_end, h->k_east_begin);
         switch (h->flow_prec) {
             case CLB_F64: CLB_EVEN(double, double); break;
             case CLB_F32: CLB_EVEN(float, float); break;
@@ -1041,14 +1039,15 @@ static void launch_flow(clb_handle* h, bool odd, int trace, int count, bool afte
 
 template <typename TS, typename TC>
 static cudaError_t launch_flow_multi(clb_handle* h, int n) {
-    GridSync* gs = (GridSync*)(h->d_err + 2);
+    GridSync* gs = (GridSync*)h->d_flow_sync;
+    uint32_t polls = (uint32_t)h->barrier_polls;
     cudaError_t e = cudaMemsetAsync(gs, 0, sizeof(GridSync), h->stream);
     if (e != cudaSuccess) return e;
     TS *f = (TS*)h->d_f, *link = (TS*)h->d_flink;
     SparseView S = view_of(h->flow_sp);
     int odd = (int)(h->flow_iters & 1);
     void* args[] = {&f, &link, &S, &h->fp, &h->d_tracer, &h->d_partials, &gs, &n, &odd, &h->k_west_end, &h->k_east_begin,
-                    &h->d_err};
+                    &polls};
     ++h->launches;
     const void* kern = h->flow_multi_one
                            ? (const void*)k_flow_multi<TS, TC, true>
@@ -1062,6 +1061,8 @@ constexpr int MULTI_STEPS = 1024, MULTI_MIN_STEPS = 3;
 
 clb_status flow_step(clb_handle* h, int n, bool trace, double eps) {
     (void)eps;
+    const clb_status ws = waits_check(h, true, false);
+    if (ws != CLB_OK) return ws;
     if (trace && h->flow_multi && !h->flow_tuned && n >= MULTI_MIN_STEPS) {
         for (int k = 0; k < n; k += MULTI_STEPS) {
             const int m = std::min(MULTI_STEPS, n - k);
@@ -1097,6 +1098,9 @@ clb_status flow_solve(clb_handle* h, int max_it, double eps, int* iterations, bo
     cudaError_t e = cudaMemcpyAsync(&cur, h->d_tracer, sizeof(Tracer), cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return cuda_check(h, e, "tracer read");
+    if (cur.gave_up) h->flow_gave_up = true;
+    clb_status waited = waits_check(h, true, false);
+    if (waited != CLB_OK) return waited;
     t0.eps = eps;
     t0.iterations = cur.iterations;
     t0.energy = cur.energy;
@@ -1119,13 +1123,15 @@ clb_status flow_solve(clb_handle* h, int max_it, double eps, int* iterations, bo
         e = cudaMemcpyAsync(&cur, h->d_tracer, sizeof(Tracer), cudaMemcpyDeviceToHost, h->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
         if (e != cudaSuccess) return cuda_check(h, e, "tracer read");
+        if (cur.gave_up) h->flow_gave_up = true;
+        if ((waited = waits_check(h, true, false)) != CLB_OK) break;
         if (cur.converged) { conv = true; break; }
         if (stream) chunk = chunk >= 32 ? 32 : chunk * 2;
         else if (chunk < 1024) chunk *= 2;
     }
     h->flow_iters = cur.iterations;  // steps after convergence were no-ops
     if (iterations) *iterations = (int)(cur.iterations - start);
-    if (keep_window) {
+    if (keep_window && waited == CLB_OK) {
         h->resolve_tracer = cur;
         h->resolve_tracer_valid = true;
     }
@@ -1133,6 +1139,7 @@ clb_status flow_solve(clb_handle* h, int max_it, double eps, int* iterations, bo
     int zero = 0;
     cudaMemcpyAsync(&h->d_tracer->converged, &zero, sizeof(int), cudaMemcpyHostToDevice, h->stream);
     cudaStreamSynchronize(h->stream);
+    if (waited != CLB_OK) return waited;
     // a diverged solve (NaN or Inf stored energy; the tracer reads a NaN window as settled) stops
     // the run cleanly, as complab.cpp:3116-3117 does
     if (!std::isfinite(cur.energy))

@@ -15,8 +15,8 @@ struct GridSync {
 // The `round`-th barrier of the launch (1, 2, ...), called by every thread of every block. What the
 // blocks wrote before it is visible after it: each block's threads meet, one of them publishes with a
 // fence and an increment, waits for the others, fences, and releases its block. False when a wait
-// gave up (about 2^24 polls, seconds); the caller then returns.
-__device__ __forceinline__ bool grid_barrier(GridSync* g, unsigned round) {
+// gave up, after `polls` looks; the caller then sets the handle's flag and returns.
+__device__ __forceinline__ bool grid_barrier(GridSync* g, unsigned round, uint32_t polls) {
     __shared__ int s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -24,7 +24,7 @@ __device__ __forceinline__ bool grid_barrier(GridSync* g, unsigned round) {
         __threadfence();
         atomicAdd(&g->arrived, 1u);
         int ok = 0;
-        for (uint32_t it = 0; it < (1u << 24); ++it) {
+        for (uint32_t it = 0; it < polls; ++it) {
             if (*(volatile unsigned*)&g->arrived >= target) {
                 ok = 1;
                 break;

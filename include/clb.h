@@ -151,6 +151,9 @@ clb_status clb_destroy(clb_handle* h);
 const char* clb_last_error(const clb_handle* h);
 /* Message of the last failure of a call that had no handle to record it in. */
 const char* clb_global_error(void);
+/* Waits for the handle's work. CLB_TIMEOUT: a bounded wait of a step gave up, which leaves its lattice
+ * undefined until clb_flow_init or clb_ade_init; besides this call, flow solves, steps, readbacks and
+ * reductions of that lattice, its coupling, batches of it, clb_run and saved checkpoints report it. */
 clb_status clb_synchronize(clb_handle* h);
 
 /* Every call of the handle enqueues on this stream (a cudaStream_t). By default the handle
@@ -175,6 +178,9 @@ clb_status clb_get_stream(clb_handle* h, void** stream);
  *                    where two slot sets per thread leave two resident CTAs per SM, i.e. up to
  *                    8 FP32 or 4 FP64 species), 0: the streamed step (default), or where an
  *                    abiotic law, a gate or a rate-law file couples the species the staged one.
+ *   "barrier_polls"  limit of one wait at the grid-wide barrier of a many-step launch, in looks at its
+ *                    counter (default 2^24, about 10 s); a wait that reaches it gives up (CLB_TIMEOUT,
+ *                    see clb_synchronize).
  * Unknown keys are an error. */
 clb_status clb_tune(clb_handle* h, const char* key, int value);
 
