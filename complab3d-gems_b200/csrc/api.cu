@@ -190,18 +190,31 @@ clb_status clb_get_stream(clb_handle* h, void** stream) {
 clb_status clb_tune(clb_handle* h, const char* key, int value) {
     if (!h || !key) return fail(h, CLB_INVALID_ARG, "null argument");
     const std::string k = key;
-    if (k.compare(0, 5, "flow_") == 0) h->flow_tuned = true;  // the per-step kernels the key chooses between
-    if (k == "flow_even_tma") { h->flow_even_tma = value ? 1 : 0; return CLB_OK; }
+    // an accepted "flow_" key takes the flow step through the per-step kernels it chooses between; a refused one
+    // changes nothing
+    if (k == "flow_streamed") {
+        CLB_ON_DEVICE(h);
+        waits_check(h, true, false, true);  // while the steps through tiles are still looked at
+        h->flow_tuned = !value;
+        return CLB_OK;
+    }
+    if (k == "flow_even_tma") {
+        h->flow_even_tma = value ? 1 : 0;
+        h->flow_tuned = true;
+        return CLB_OK;
+    }
     if (k == "ade_pipe") { h->ade_pipe = value ? 1 : 0; return CLB_OK; }
     if (k == "flow_odd_pipe") {
         if (value && h->flow_ready && !h->flow_pipe_grid)
             return fail(h, CLB_INVALID_ARG, "flow_odd_pipe needs 4- or 8-byte flow storage");
         h->flow_odd_pipe = value ? 1 : 0;
+        h->flow_tuned = true;
         return CLB_OK;
     }
     if (k == "flow_min_blocks") {
         if (value != 2 && value != 3) return fail(h, CLB_INVALID_ARG, "flow_min_blocks is 2 or 3");
         h->flow_minb = value;
+        h->flow_tuned = true;
         return CLB_OK;
     }
     if (k == "barrier_polls") {

@@ -164,7 +164,8 @@ clb_status clb_get_stream(clb_handle* h, void** stream);
 
 /* Launch-shape and kernel-variant knobs (used by the autotuner). By default every flow and transport
  * step is streamed (one node per thread, no staging; many steps per launch on small lattices where
- * that is faster); setting any "flow_" key takes the flow steps through the kernels it names:
+ * that is faster); a "flow_" key that is accepted takes the flow steps through the kernels it names:
+ *   "flow_streamed"  1: back to the default, 0: the kernels the other keys name;
  *   "flow_even_tma"  1: even AA step through shared-memory tiles and bulk copies,
  *                    0: the plain per-thread load/store step;
  *   "flow_min_blocks" 2 or 3: resident CTAs per SM the gather/scatter step is compiled for
