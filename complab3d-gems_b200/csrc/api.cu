@@ -27,7 +27,7 @@ clb_status cuda_check(clb_handle* h, cudaError_t e, const char* what) {
 }
 
 clb_status waits_check(clb_handle* h, bool flow, bool ade, bool look) {
-    if (flow && look && h->flow_tuned && h->d_tracer) {
+    if (flow && look && (h->flow_keyed || h->flow_tuned) && h->d_tracer) {
         int gave_up = 0;
         const cudaError_t e = copy_on_stream(h, &gave_up, &h->d_tracer->gave_up, sizeof(int), cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) return cuda_check(h, e, "tracer read");
@@ -195,12 +195,13 @@ clb_status clb_tune(clb_handle* h, const char* key, int value) {
     if (k == "flow_streamed") {
         CLB_ON_DEVICE(h);
         waits_check(h, true, false, true);  // while the steps through tiles are still looked at
-        h->flow_tuned = !value;
+        h->flow_keyed = !value;
+        h->flow_tuned = false;
         return CLB_OK;
     }
     if (k == "flow_even_tma") {
         h->flow_even_tma = value ? 1 : 0;
-        h->flow_tuned = true;
+        h->flow_keyed = true;
         return CLB_OK;
     }
     if (k == "ade_pipe") { h->ade_pipe = value ? 1 : 0; return CLB_OK; }
@@ -208,13 +209,13 @@ clb_status clb_tune(clb_handle* h, const char* key, int value) {
         if (value && h->flow_ready && !h->flow_pipe_grid)
             return fail(h, CLB_INVALID_ARG, "flow_odd_pipe needs 4- or 8-byte flow storage");
         h->flow_odd_pipe = value ? 1 : 0;
-        h->flow_tuned = true;
+        h->flow_keyed = true;
         return CLB_OK;
     }
     if (k == "flow_min_blocks") {
         if (value != 2 && value != 3) return fail(h, CLB_INVALID_ARG, "flow_min_blocks is 2 or 3");
         h->flow_minb = value;
-        h->flow_tuned = true;
+        h->flow_keyed = true;
         return CLB_OK;
     }
     if (k == "barrier_polls") {

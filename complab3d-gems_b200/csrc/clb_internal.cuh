@@ -266,7 +266,8 @@ struct clb_handle_s {
     int flow_odd_pipe = 1;            // odd step pipelined through shared memory (4- and 8-byte storage)
     int flow_multi = 0;               // blocks of the many-step launch of a small lattice; 0: one launch per step
     bool flow_multi_one = false;      // its threads keep one node each
-    bool flow_tuned = false;          // a per-step kernel variant was asked for (clb_tune) or measured faster
+    bool flow_keyed = false;          // a key (clb_tune) asked for the per-step kernels: every flow step
+    bool flow_tuned = false;          // clb_autotune measured them faster: steps without the tracer, as it timed
     int flow_pipe_grid = 0;           // its resident-CTA grid; 0 where it is not available
     int* d_flow_sync = nullptr;       // grid-wide barrier of the many-step flow launches (GridSync)
     int barrier_polls = 1 << 24;      // limit of one wait at a grid-wide barrier (about 10 s); "barrier_polls"

@@ -957,10 +957,11 @@ clb_status flow_init(clb_handle* h, double delta_p) {
     return cuda_check(h, cudaGetLastError(), "flow init");
 }
 
-// The streamed step, except where a tuning key selects the tiled and pipelined kernels. A traced step is two
+// The streamed step, except where a tuning key selects the tiled and pipelined kernels or clb_autotune
+// measured them faster for steps without the tracer. A traced step is two
 // chained launches, the step and its energy (tiled and pipelined kernels -> streamed, us per traced step: 480 k
 // nodes FP32 23.1 -> 22.4, 1.3 M 55.5 -> 54.5, 3.8 M 153.6 -> 147.4; FP64 3.8 M 261 -> 237, FP16 174 -> 124).
-static bool flow_streams(const clb_handle* h) { return !h->flow_tuned; }
+static bool flow_streams(const clb_handle* h, bool trace) { return !h->flow_keyed && (trace || !h->flow_tuned); }
 
 // One step. The streamed step forms the stored energy, and counts `count` iterations, only where count is
 // not 0; the kernels a tuning key selects do both at every step.
@@ -969,7 +970,7 @@ static void launch_flow(clb_handle* h, bool odd, int trace, int count, bool afte
     const FlowParams& P = h->fp;
     const SparseView S = view_of(h->flow_sp);
     const int grid = h->flow_grid;
-    if (flow_streams(h)) {
+    if (flow_streams(h, trace != 0)) {
         const unsigned g = (unsigned)std::max<int64_t>(1, flow_tiles(h));
         auto go = [&](auto kern, auto* ts) {
             using TS = std::remove_pointer_t<decltype(ts)>;
@@ -1063,7 +1064,7 @@ clb_status flow_step(clb_handle* h, int n, bool trace, double eps) {
     (void)eps;
     const clb_status ws = waits_check(h, true, false);
     if (ws != CLB_OK) return ws;
-    if (trace && h->flow_multi && !h->flow_tuned && n >= MULTI_MIN_STEPS) {
+    if (trace && h->flow_multi && !h->flow_keyed && n >= MULTI_MIN_STEPS) {
         for (int k = 0; k < n; k += MULTI_STEPS) {
             const int m = std::min(MULTI_STEPS, n - k);
             cudaError_t e;
@@ -1078,7 +1079,7 @@ clb_status flow_step(clb_handle* h, int n, bool trace, double eps) {
         return CLB_OK;
     }
     for (int k = 0; k < n; ++k) {
-        launch_flow(h, (h->flow_iters & 1) != 0, trace ? 1 : 0, trace ? 1 : (k + 1 == n ? n : 0), k > 0 && flow_streams(h));
+        launch_flow(h, (h->flow_iters & 1) != 0, trace ? 1 : 0, trace ? 1 : (k + 1 == n ? n : 0), k > 0 && flow_streams(h, trace));
         h->flow_iters += 1;
     }
     return cuda_check(h, cudaGetLastError(), "flow step");
@@ -1112,7 +1113,7 @@ clb_status flow_solve(clb_handle* h, int max_it, double eps, int* iterations, bo
     // decision before its stores, which saves every other step a round trip), so the run up to a full
     // window goes at once and then few at a time: the wait costs about 15 us, a step of a lattice that
     // takes the streamed kernel 16 us and more. The other kernels return at once.
-    const bool multi = h->flow_multi && !h->flow_tuned, stream = !multi && flow_streams(h);
+    const bool multi = h->flow_multi && !h->flow_keyed, stream = !multi && flow_streams(h, true);
     int chunk = multi ? MULTI_STEPS : stream ? std::max(4, TRACER_WINDOW - t0.count) : 64;
     bool conv = false;
     while (done < max_it) {
@@ -1305,10 +1306,11 @@ clb_status flow_stats(clb_handle* h, double char_length, clb_flow_stats* out) {
     return CLB_OK;
 }
 
-// Times every kernel variant (the default: many steps per launch where the lattice is small enough for
-// it, else the streamed step; even step through TMA tiles or not; odd step compiled for 2 or 3
-// resident CTAs, or pipelined through shared memory) over `steps` steps and keeps the fastest. The lattice state is saved before
-// and restored after, so the run is unchanged. Writes a one-line report into `report`.
+// Times the kernels of a step without the tracer (the default, the streamed step; even step through TMA tiles or
+// not with the odd step compiled for 2 or 3 resident CTAs or pipelined through shared memory) over `steps`
+// steps and keeps the fastest for such steps; a solve's, which are traced and on a small lattice go many to a
+// launch, keep theirs. A key's choice before it lapses. The lattice state is saved before and restored
+// after, so the run is unchanged. Writes a one-line report into `report`.
 clb_status flow_autotune(clb_handle* h, int steps, char* report, int report_len) {
     if (steps < 2) steps = 2;
     steps += steps & 1;
@@ -1342,7 +1344,7 @@ clb_status flow_autotune(clb_handle* h, int steps, char* report, int report_len)
         cudaEventElapsedTime(&ms, a, b);
         return ms;
     };
-    h->flow_tuned = false;
+    h->flow_keyed = h->flow_tuned = false;
     const float base = timed();
     {
         char buf[64];

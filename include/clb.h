@@ -185,8 +185,8 @@ clb_status clb_get_stream(clb_handle* h, void** stream);
  * Unknown keys are an error. */
 clb_status clb_tune(clb_handle* h, const char* key, int value);
 
-/* Times the default and every kernel variant of the flow step over `steps` steps on this domain and keeps the
- * fastest; the lattice state is saved and restored, so the simulation is unchanged. A one-line
+/* Times the default and every kernel variant of the flow step without the solve's tracer over `steps` steps on
+ * this domain and keeps the fastest for such steps (a solve keeps its default); an earlier "flow_" key lapses. The lattice state is saved and restored, so the simulation is unchanged. A one-line
  * report of the timings is written to `report` (may be NULL). */
 clb_status clb_autotune(clb_handle* h, int steps, char* report, int report_len);
 

@@ -52,3 +52,20 @@ def test_an_accepted_key_changes_the_route_and_one_restores_it(clb, key, value):
     np.testing.assert_array_equal(A.flow_populations(), B.flow_populations())
     assert not many_steps_per_launch(clb, A)
     assert many_steps_per_launch(clb, B)
+
+
+@pytest.mark.parametrize("key", [None, "flow_even_tma"])
+def test_autotune_leaves_the_solve_to_its_default(clb, key):
+    """The autotuner times steps without the tracer, so whatever it chooses for them a solve goes many steps to
+    a launch; the lattice is as it was."""
+    A, B = domain(clb), domain(clb)
+    for D in (A, B):
+        D.flow_step(3)
+    if key:
+        A.tune(key, 1)
+    assert "stream:" in A.autotune(8)
+    np.testing.assert_array_equal(A.flow_populations(), B.flow_populations())
+    for D in (A, B):
+        D.flow_step(5)
+    np.testing.assert_array_equal(A.flow_populations(), B.flow_populations())
+    assert many_steps_per_launch(clb, A)
