@@ -363,7 +363,7 @@ constexpr int ade_minb() {
 // (slot offsets, then every species' incoming populations, the node's velocity and biomass into
 // the calling thread's shared-memory frame F, by asynchronous copies where the element is 4 or
 // 8 bytes) and ade_finish (boundary completion, kinetics, collision, deposit, scatter). Shared by
-// the single-domain, the pipelined and the batched steps.
+// the single-domain and the pipelined step and the persistent schedule of a batch.
 //
 // Both AA steps are in-place permutations of 7 storage slots per node that every species shares:
 // incoming j is read from slot j and outgoing opp(j) is written back to slot j. Even step: slot j is

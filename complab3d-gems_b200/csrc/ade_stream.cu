@@ -315,8 +315,8 @@ bool launch_ade_multi(clb_handle* h, int steps, cudaError_t& e) {
 
 // ------------------------------------------------------------------ a batch of domains
 
-// One block per tile of the batch's table: the tile's domain goes to shared memory, then the block
-// walks the tile 128 nodes at a time. 96 uneven domains of 3 FP32 Monod species (2.9 M nodes): 138 us
+// One block per tile of the batch's table, one thread per node of it: the tile's domain goes to shared
+// memory, then the nodes are stepped. 96 uneven domains of 3 FP32 Monod species (2.9 M nodes): 138 us
 // per step where the staged form (persistent blocks over runs of the table) took 198.
 template <typename TS, typename TC, bool ODD, int U, int LAW>
 __global__ void __launch_bounds__(STREAM_THREADS, (stream_blocks<TC, U>()))

@@ -590,7 +590,7 @@ clb_status batch_schedule(clb_batch* b, int persistent, int tile, int lag, int s
         b->resident = batch_persistent_resident(prec, b->nm, ctas_per_sm);
     }
     if (persistent == 2 && b->has_flow && b->flow_prec == CLB_F16S)
-        return bfail(b, CLB_INVALID_ARG, "schedule: the staged flow step needs 4- or 8-byte flow storage");
+        return bfail(b, CLB_INVALID_ARG, "schedule: mode 2 (the launches of mode 0) is for 4- or 8-byte flow storage");
     b->persistent = persistent == 1;
     b->flow_staged = persistent == 2;
     drop_graphs(b);

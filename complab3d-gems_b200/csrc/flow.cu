@@ -749,9 +749,6 @@ __global__ void k_flow_vstats(const double* __restrict__ u, const Geom G, double
 
 // ------------------------------------------------------------------ host side
 
-
-// ------------------------------------------------------------------ host side
-
 static int64_t flow_tiles(const clb_handle* h) { return (h->flow_sp.K + STREAM_FLOW_THREADS - 1) / STREAM_FLOW_THREADS; }
 
 static size_t storage_size(int prec) { return prec == CLB_F64 ? 8 : (prec == CLB_F32 ? 4 : 2); }
