@@ -270,7 +270,7 @@ struct clb_handle_s {
     bool flow_tuned = false;          // clb_autotune measured them faster: steps without the tracer, as it timed
     int flow_pipe_grid = 0;           // its resident-CTA grid; 0 where it is not available
     int* d_flow_sync = nullptr;       // grid-wide barrier of the many-step flow launches (GridSync)
-    int barrier_polls = 1 << 24;      // limit of one wait at a grid-wide barrier (about 10 s); "barrier_polls"
+    int barrier_polls = 1 << 24;      // limit of one wait at a grid-wide barrier (seconds); "barrier_polls"
     uint8_t* d_bflag = nullptr;       // [K] species-lattice nodes where biomass may act (AdeParams::bflag)
     bool flow_gave_up = false;        // a flow step's bounded wait did (the tracer's flag, seen by the host)
     int* h_flags = nullptr;           // host-mapped pinned flags the transport steps set (enum AdeFlag)

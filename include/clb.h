@@ -180,7 +180,7 @@ clb_status clb_get_stream(clb_handle* h, void** stream);
  *                    8 FP32 or 4 FP64 species), 0: the streamed step (default), or where an
  *                    abiotic law, a gate or a rate-law file couples the species the staged one.
  *   "barrier_polls"  limit of one wait at the grid-wide barrier of a many-step launch, in looks at its
- *                    counter (default 2^24, about 10 s); a wait that reaches it gives up (CLB_TIMEOUT,
+ *                    counter (default 2^24, seconds); a wait that reaches it gives up (CLB_TIMEOUT,
  *                    see clb_synchronize).
  * Unknown keys are an error. */
 clb_status clb_tune(clb_handle* h, const char* key, int value);
