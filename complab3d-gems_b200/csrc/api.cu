@@ -230,7 +230,8 @@ clb_status clb_autotune(clb_handle* h, int steps, char* report, int report_len) 
     if (!h) return fail(nullptr, CLB_INVALID_ARG, "null handle");
     CLB_ON_DEVICE(h);
     if (!h->flow_ready) return fail(h, CLB_NOT_INITIALIZED, "clb_flow_init first");
-    return flow_autotune(h, steps, report, report_len);
+    const clb_status ws = waits_check(h, true, false, true);  // else it would time steps that are refused
+    return ws != CLB_OK ? ws : flow_autotune(h, steps, report, report_len);
 }
 
 clb_status clb_flow_init(clb_handle* h, double delta_p) {

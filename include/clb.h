@@ -152,8 +152,8 @@ const char* clb_last_error(const clb_handle* h);
 /* Message of the last failure of a call that had no handle to record it in. */
 const char* clb_global_error(void);
 /* Waits for the handle's work. CLB_TIMEOUT: a bounded wait of a step gave up, which leaves its lattice
- * undefined until clb_flow_init or clb_ade_init; besides this call, flow solves, steps, readbacks and
- * reductions of that lattice, its coupling, batches of it, clb_run and saved checkpoints report it. */
+ * undefined until clb_flow_init or clb_ade_init; besides this call, flow solves, steps, readbacks,
+ * reductions and the autotuning of that lattice, its coupling, batches of it, clb_run and saved checkpoints report it. */
 clb_status clb_synchronize(clb_handle* h);
 
 /* Every call of the handle enqueues on this stream (a cudaStream_t). By default the handle

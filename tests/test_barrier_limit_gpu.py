@@ -38,7 +38,7 @@ def test_flow_solve_reports_a_barrier_that_gave_up(clb, tmp_path):
     times_out(clb, D.flow_solve, 3000, 1e-9)
     D.tune("barrier_polls", DEFAULT)
     for call, args in ((D.flow_solve, (3000, 1e-9)), (D.flow_step, (1,)), (D.velocity, ()), (D.flow_populations, ()),
-                       (D.flow_stats, ()), (D.couple_velocity, ()), (D.checkpoint_save, (str(tmp_path / "c"),)), (D.sync, ())):
+                       (D.flow_stats, ()), (D.autotune, (8,)), (D.couple_velocity, ()), (D.checkpoint_save, (str(tmp_path / "c"),)), (D.sync, ())):
         times_out(clb, call, *args)
     D.ade_step(4)  # the species lattices are not concerned
     D.concentration(0)
